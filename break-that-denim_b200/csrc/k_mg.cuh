@@ -119,77 +119,90 @@ __device__ __forceinline__ float weightOf(int i, int I, int n) {
 }
 __device__ __forceinline__ float pwSlot(float4 w, int s) { return s == 0 ? w.x : s == 1 ? w.y : s == 2 ? w.z : w.w; }
 
-constexpr int RAP_THREADS = 64;
+constexpr int RAP_NODES = 8;
 
 // Galerkin coarse row P^T A P of coarse node I (rap, multigrid.wgsl:115-178; galerkin,
-// newtonMultigrid.ts:345-387). One thread per coarse node; its 25 accumulators live in shared memory.
+// newtonMultigrid.ts:345-387): a warp a node, lane o on the block of stencil offset o (25 of the 32 lanes),
+// eight nodes a CTA. The lane gathers its block's terms wa A_ab wb over the fine nodes a of I and b of its
+// coarse neighbour in the row's order. It is bound by the latency of those loads (L2), not by bytes or
+// FLOPs: one thread a node with its 25 accumulators in shared memory had 25 times fewer of them in flight
+// (and, scattering each A_ab to up to four accumulators, summed in the same order).
 template <class Rows>
-__global__ void __launch_bounds__(RAP_THREADS) k_rap(DLevel F, DLevel C) {
-  __shared__ float acc[RAP_THREADS][153];  // odd stride: conflict-free per-thread rows
-  int I = blockIdx.x * blockDim.x + threadIdx.x;
-  if (I >= C.N) return;
-  float* a25 = acc[threadIdx.x];
-  for (int q = 0; q < 150; ++q) a25[q] = 0.f;
+__global__ void __launch_bounds__(32 * RAP_NODES) k_rap(DLevel F, DLevel C) {
+  __shared__ __align__(16) float rows[RAP_NODES][4 * COARSE_PLANES];
+  __shared__ float sW[RAP_NODES][9][32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, I0 = blockIdx.x * RAP_NODES;
+  const int I = min(I0 + warp, C.N - 1);
   int ci, cj, l;
-  nodeCoord(C, I, &ci, &cj, &l);
-  const DLevelLayer Lf = F.layers[l];
+  nodeAt(C, I, &ci, &cj, &l);
+  const DLevelLayer Lf = layerOf(F, l), Lc = layerOf(C, l);
   const int nxf = Lf.nx, nyf = Lf.ny;
+  const int Ji = ci + lane % 5 - 2, Jj = cj + lane / 5 - 2;  // the lane's coarse neighbour
+  const bool on = lane < 25 && Ji >= 0 && Jj >= 0 && Ji < Lc.nx && Jj < Lc.ny;
+  const int bi0 = coarseToFine(Ji, nxf), bj0 = coarseToFine(Jj, nyf);
   const int fi0 = coarseToFine(ci, nxf), fj0 = coarseToFine(cj, nyf);
-  for (int aj = fj0 - 1; aj <= fj0 + 1; ++aj) {
-    if (aj < 0 || aj >= nyf) continue;
-    if (weightOf(aj, cj, nyf) == 0.f) continue;
-    for (int ai = fi0 - 1; ai <= fi0 + 1; ++ai) {
-      if (ai < 0 || ai >= nxf) continue;
-      if (weightOf(ai, ci, nxf) == 0.f) continue;
-      int a = levelNode(Lf, ai, aj);
-      if (F.fixed[a]) continue;
-      Bracket bai = bracketOf(ai, nxf), baj = bracketOf(aj, nyf);
-      float wa = pwSlot(F.pw[a], (bai.lo == ci ? 0 : 1) + 2 * (baj.lo == cj ? 0 : 1));
-      if (wa == 0.f) continue;
-      for (int k = 0; k <= Rows::NC; ++k) {
-        int2 off = make_int2(0, 0);
-        Sym Ab;
-        if (k == Rows::NC) {
-          Ab = Rows::diag(F.op, F.N, a);
-        } else {
-          off = Rows::offset(k);
-          Ab = Rows::coupling(F.op, F.N, a, k);
-        }
-        if (symIsZero(Ab)) continue;
-        int bi = ai + off.x, bj = aj + off.y;
-        if (bi < 0 || bj < 0 || bi >= nxf || bj >= nyf) continue;
-        Bracket bri = bracketOf(bi, nxf), brj = bracketOf(bj, nyf);
-        float4 wb = F.pw[levelNode(Lf, bi, bj)];
-        for (int kj = 0; kj < 2; ++kj) {
-          int J = kj ? brj.hi : brj.lo;
-          for (int ki = 0; ki < 2; ++ki) {
-            int Ii = ki ? bri.hi : bri.lo;
-            float wJ = pwSlot(wb, ki + 2 * kj);
-            if (wJ == 0.f) continue;
-            const int oj = J - cj + 2, oi = Ii - ci + 2;
-            if ((unsigned)oj > 4u || (unsigned)oi > 4u) continue;  // radius-2 closure (galerkin throws there)
-            int o = oj * 5 + oi;
-            float s = wa * wJ;
-            float* p = a25 + 6 * o;
-            p[0] += Ab.xx * s, p[1] += Ab.xy * s, p[2] += Ab.xz * s, p[3] += Ab.yy * s, p[4] += Ab.yz * s, p[5] += Ab.zz * s;
-          }
-        }
+  Sym acc = symZero();
+  // the weights of the neighbour's support, the 3 x 3 fine nodes around (bi0, bj0), a lane's own in sW
+#pragma unroll
+  for (int p = 0; p < 9; ++p) {
+    const int bi = bi0 - 1 + p % 3, bj = bj0 - 1 + p / 3;
+    float w = 0.f;
+    if (on && bi >= 0 && bj >= 0 && bi < nxf && bj < nyf) {
+      const Bracket u = bracketOf(bi, nxf), v = bracketOf(bj, nyf);
+      const int ki = u.lo == Ji ? 0 : u.hi == Ji ? 1 : -1, kj = v.lo == Jj ? 0 : v.hi == Jj ? 1 : -1;
+      if (ki >= 0 && kj >= 0) w = pwSlot(F.pw[levelNode(Lf, bi, bj)], ki + 2 * kj);
+    }
+    sW[warp][p][lane] = w;
+  }
+  __syncwarp();
+  // fine node (bi, bj)'s weight to the neighbour, 0 outside its support
+  auto weight = [&](int bi, int bj) {
+    const int u = bi - bi0 + 1, v = bj - bj0 + 1;
+    return (unsigned)u < 3u && (unsigned)v < 3u ? sW[warp][3 * v + u][lane] : 0.f;
+  };
+  auto add = [&](const Sym& A, float s) {
+    acc.xx += A.xx * s, acc.xy += A.xy * s, acc.xz += A.xz * s, acc.yy += A.yy * s, acc.yz += A.yz * s, acc.zz += A.zz * s;
+  };
+  for (int q = 0; q < 9; ++q) {
+    const int ai = fi0 - 1 + q % 3, aj = fj0 - 1 + q / 3;
+    if (ai < 0 || aj < 0 || ai >= nxf || aj >= nyf) continue;
+    if (weightOf(ai, ci, nxf) == 0.f || weightOf(aj, cj, nyf) == 0.f) continue;
+    const int a = levelNode(Lf, ai, aj);
+    if (F.fixed[a]) continue;
+    const Bracket bai = bracketOf(ai, nxf), baj = bracketOf(aj, nyf);
+    const float wa = pwSlot(F.pw[a], (bai.lo == ci ? 0 : 1) + 2 * (baj.lo == cj ? 0 : 1));
+    if (wa == 0.f || !on) continue;
+    if constexpr (Rows::NC == 24) {
+      // the couplings in offset order: b over the neighbour's support, a itself last
+#pragma unroll
+      for (int p = 0; p < 9; ++p) {
+        const int bi = bi0 - 1 + p % 3, bj = bj0 - 1 + p / 3, di = bi - ai, dj = bj - aj;
+        if (di < -2 || di > 2 || dj < -2 || dj > 2 || (di == 0 && dj == 0)) continue;
+        const float wb = weight(bi, bj);
+        if (wb != 0.f) add(coarseBlock(F.op, F.N, a, (dj + 2) * 5 + di + 2), wa * wb);
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < Rows::NC; ++k) {
+        const int2 off = Rows::offset(k);
+        const float wb = weight(ai + off.x, aj + off.y);
+        if (wb != 0.f) add(Rows::coupling(F.op, F.N, a, k), wa * wb);
       }
     }
+    const float wb = weight(ai, aj);
+    if (wb != 0.f) add(Rows::diag(F.op, F.N, a), wa * wb);
   }
-  const float* c = a25 + 6 * 12;
-  bool fixedRow = c[0] + c[3] + c[5] <= 0.f;
-  if (fixedRow) {
-    for (int q = 0; q < 150; ++q) a25[q] = 0.f;
-    a25[72] = 1.f, a25[75] = 1.f, a25[77] = 1.f;
+  const float trace = __shfl_sync(0xffffffffu, acc.xx + acc.yy + acc.zz, 12);
+  const bool fixedRow = trace <= 0.f;
+  if (fixedRow) acc = lane == 12 ? symId(1.f) : symZero();
+  if (lane < 25) storeSymAt(rows[warp], 6 * lane, acc);
+  if (lane == 25) rows[warp][150] = rows[warp][151] = 0.f;
+  if (lane == 0 && I0 + warp < C.N) C.fixed[I] = fixedRow ? 1u : 0u;
+  __syncthreads();
+  for (int e = threadIdx.x; e < COARSE_PLANES * RAP_NODES; e += 32 * RAP_NODES) {
+    const int p = e / RAP_NODES, w = e % RAP_NODES;
+    if (I0 + w < C.N) C.op[(size_t)p * C.N + I0 + w] = *reinterpret_cast<const float4*>(&rows[w][4 * p]);
   }
-  for (int p = 0; p < COARSE_PLANES; ++p) {
-    float v[4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) v[q] = 4 * p + q < 150 ? a25[4 * p + q] : 0.f;
-    C.op[(size_t)p * C.N + I] = make_float4(v[0], v[1], v[2], v[3]);
-  }
-  C.fixed[I] = fixedRow ? 1u : 0u;
 }
 
 // r = b - A x on the fine level (residual, multigrid.wgsl:182-199); fixed rows give 0. Loads are

@@ -428,10 +428,10 @@ struct btd_solver {
       DLevel F = levels[k].dev(), Cl = levels[k + 1].dev();
       if (k == 0) {
         k_prolong_weights<FineRows, true><<<blocksFor(F.N, 128), 128, 0, s>>>(F, segs);
-        k_rap<FineRows><<<blocksFor(Cl.N, RAP_THREADS), RAP_THREADS, 0, s>>>(F, Cl);
+        k_rap<FineRows><<<blocksFor(Cl.N, RAP_NODES), 32 * RAP_NODES, 0, s>>>(F, Cl);
       } else {
         k_prolong_weights<CoarseRows, false><<<blocksFor(F.N, 128), 128, 0, s>>>(F, segs);
-        k_rap<CoarseRows><<<blocksFor(Cl.N, RAP_THREADS), RAP_THREADS, 0, s>>>(F, Cl);
+        k_rap<CoarseRows><<<blocksFor(Cl.N, RAP_NODES), 32 * RAP_NODES, 0, s>>>(F, Cl);
       }
       encFactor(s, (int)k + 1);
     }
