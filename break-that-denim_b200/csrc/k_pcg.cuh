@@ -38,6 +38,17 @@ __device__ bool gridReduce(const Reduce& R, double (&v)[NV], double (&out)[NV]) 
     if (lane == 0) wsum[warp][q] = s;
   }
   __syncthreads();
+  if (gridDim.x == 1) {  // one block (256 nodes and fewer): its sum is the total, no round trip through memory
+    if (threadIdx.x == 0) {
+#pragma unroll
+      for (int q = 0; q < NV; ++q) {
+        double s = 0;
+        for (int w = 0; w < RED_THREADS / 32; ++w) s += wsum[w][q];
+        out[q] = s;
+      }
+    }
+    return true;
+  }
   if (threadIdx.x == 0) {
 #pragma unroll
     for (int q = 0; q < NV; ++q) {
@@ -75,7 +86,8 @@ __device__ bool gridReduce(const Reduce& R, double (&v)[NV], double (&out)[NV]) 
 
 struct PcgArgs {
   DLevel F;  // fine level: B = r, X = z
-  float4* p;
+  float4* p;   // the direction of even iterations
+  float4* p1;  // and of odd ones (k_pcg_matvec reads the one before from the other)
   float4* Ap;
   float4* delta;
   float4* b0;  // the right-hand side PCG started from (the true residual's b)
@@ -122,13 +134,6 @@ __global__ void __launch_bounds__(RED_THREADS) k_pcg_init(PcgArgs a) {
     s.check = 0;
     s.restart = 0;
   }
-}
-
-// Symmetric fp32 block times an FP64 vector, in FP64.
-__device__ __forceinline__ void symVecAddD(const Sym& A, const double* x, double& y0, double& y1, double& y2) {
-  y0 += (double)A.xx * x[0] + (double)A.xy * x[1] + (double)A.xz * x[2];
-  y1 += (double)A.xy * x[0] + (double)A.yy * x[1] + (double)A.yz * x[2];
-  y2 += (double)A.xz * x[0] + (double)A.yz * x[1] + (double)A.zz * x[2];
 }
 
 // y += (row n of the operator PCG solves with) x, in FP64: the FP64 row when there is one, else the fp32
@@ -236,48 +241,41 @@ __global__ void __launch_bounds__(RED_THREADS) k_pcg_dot_rz(PcgArgs a, int first
   }
 }
 
-// p = z + beta p (first: p = z).
-__global__ void k_pcg_update_p(PcgArgs a, int first) {
-  pdlWait();
-  pdlLaunchNext();
-  int n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= a.F.N) return;
-  float3 z = f3(a.F.X[n]);
-  if (first) {
-    a.p[n] = make_float4(z.x, z.y, z.z, 0.f);
-    return;
-  }
-  float beta = (float)a.scal->beta;
-  float3 p = z + beta * f3(a.p[n]);
-  a.p[n] = make_float4(p.x, p.y, p.z, 0.f);
-}
-
-// Ap = A p (fixed rows 0), p . Ap; alpha = rz / pAp (0 and stop when pAp <= 0, as pcg() breaks).
-__global__ void __launch_bounds__(RED_THREADS) k_pcg_matvec(PcgArgs a) {
+// p = z + beta p (first: p = z); Ap = A p (fixed rows 0), p . Ap; alpha = rz / pAp (0 and stop when
+// pAp <= 0, as pcg() breaks). Each node forms its neighbours' p as they do (one launch and one pass over p
+// less than an update of its own), so the new p goes to the other of two buffers.
+__global__ void __launch_bounds__(RED_THREADS) k_pcg_matvec(PcgArgs a, int first) {
   pdlWait();
   pdlLaunchNext();
   double v[1] = {0.0};
   const DLevel& F = a.F;
+  const bool odd = (a.scal->pcgIt & 1) != 0;
+  float4* pNew = odd ? a.p1 : a.p;
+  const float4* pOld = odd ? a.p : a.p1;
+  const float beta = first ? 0.f : (float)a.scal->beta;
+  auto direction = [&](int m) {
+    const float3 z = f3(F.X[m]);
+    return first ? z : z + beta * f3(pOld[m]);
+  };
   for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < F.N; n += gridDim.x * blockDim.x) {
     // the row's loads do not wait for its fixed flag (a fixed row's product is dropped)
     float3 y = make_float3(0, 0, 0);
     const uint32_t fixedRow = F.fixed[n];
-    {
-      // products summed in FP64: the recurrence residual then drifts from the true one by the rounding
-      // of the stored Ap only
-      double y0 = 0.0, y1 = 0.0, y2 = 0.0;
-      pcgRowApply(
-          a, n,
-          [&](int m, double* q) {
-            const float4 pm = a.p[m];
-            q[0] = pm.x, q[1] = pm.y, q[2] = pm.z;
-            return true;
-          },
-          y0, y1, y2);
-      if (!fixedRow) y = make_float3((float)y0, (float)y1, (float)y2);
-    }
+    // products summed in FP64: the recurrence residual then drifts from the true one by the rounding of the
+    // stored Ap only
+    double y0 = 0.0, y1 = 0.0, y2 = 0.0;
+    float3 p;
+    pcgRowGather<float>(
+        F, a.op64, n,
+        [&](int m, float* q) {
+          const float3 pm = direction(m);
+          if (m == n) p = pm;
+          q[0] = pm.x, q[1] = pm.y, q[2] = pm.z;
+        },
+        y0, y1, y2);
+    if (!fixedRow) y = make_float3((float)y0, (float)y1, (float)y2);
+    pNew[n] = make_float4(p.x, p.y, p.z, 0.f);
     a.Ap[n] = make_float4(y.x, y.y, y.z, 0.f);
-    float3 p = f3(a.p[n]);
     v[0] += (double)y.x * p.x + (double)y.y * p.y + (double)y.z * p.z;
   }
   double out[1];
@@ -312,8 +310,9 @@ __global__ void __launch_bounds__(RED_THREADS) k_pcg_update_xr(PcgArgs a) {
   double v[1] = {0.0};
   const double alphaD = a.scal->alpha;
   const float alpha = (float)alphaD;
+  const float4* p = (a.scal->pcgIt & 1) ? a.p1 : a.p;
   for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < a.F.N; n += gridDim.x * blockDim.x) {
-    const float3 pn = f3(a.p[n]);
+    const float3 pn = f3(p[n]);
     const double d0 = a.dd[3 * n] + alphaD * pn.x, d1 = a.dd[3 * n + 1] + alphaD * pn.y, d2 = a.dd[3 * n + 2] + alphaD * pn.z;
     a.dd[3 * n] = d0, a.dd[3 * n + 1] = d1, a.dd[3 * n + 2] = d2;
     float3 r = f3(a.F.B[n]) - alpha * f3(a.Ap[n]);
@@ -365,13 +364,8 @@ __global__ void __launch_bounds__(RED_THREADS) k_pcg_true_residual(PcgArgs a) {
     const float3 b = f3(a.b0[n]);
     double y0 = 0.0, y1 = 0.0, y2 = 0.0;
     const uint32_t fixedRow = F.fixed[n];
-    pcgRowApply(
-        a, n,
-        [&](int m, double* q) {
-          q[0] = a.dd[3 * m], q[1] = a.dd[3 * m + 1], q[2] = a.dd[3 * m + 2];
-          return true;
-        },
-        y0, y1, y2);
+    pcgRowGather<double>(
+        F, a.op64, n, [&](int m, double* q) { q[0] = a.dd[3 * m], q[1] = a.dd[3 * m + 1], q[2] = a.dd[3 * m + 2]; }, y0, y1, y2);
     if (fixedRow) y0 = y1 = y2 = 0.0;
     const double r0 = (double)b.x - y0, r1 = (double)b.y - y1, r2 = (double)b.z - y2;
     a.F.B[n] = make_float4((float)r0, (float)r1, (float)r2, 0.f);

@@ -168,7 +168,7 @@ struct btd_solver {
   unsigned* dTicket = nullptr;
   NodeStatic* dNodes = nullptr;
   DLayer* dLayers = nullptr;
-  float4 *x = nullptr, *v = nullptr, *dx = nullptr, *pred = nullptr, *ext = nullptr, *delta = nullptr, *p = nullptr,
+  float4 *x = nullptr, *v = nullptr, *dx = nullptr, *pred = nullptr, *ext = nullptr, *delta = nullptr, *p = nullptr, *p1 = nullptr,
          *Ap = nullptr, *b0 = nullptr;
   double* deltaD = nullptr;
   // the fine operator in FP64, the operator PCG solves with (null when the solve takes the fp32 rows)
@@ -322,6 +322,7 @@ struct btd_solver {
     PcgArgs a;
     a.F = levels[0].dev();
     a.p = p;
+    a.p1 = p1;
     a.Ap = Ap;
     a.delta = delta;
     a.b0 = b0;
@@ -553,8 +554,7 @@ struct btd_solver {
   void encPcgBody(cudaStream_t s, const PcgArgs& a) {
     encVCycle(s, 0);
     launch(k_pcg_dot_rz, redBlocks, RED_THREADS, 0, s, a, 0);
-    launch(k_pcg_update_p, blocksFor(N, 256), 256, 0, s, a, 0);
-    launch(k_pcg_matvec, redBlocks, RED_THREADS, 0, s, a);
+    launch(k_pcg_matvec, redBlocks, RED_THREADS, 0, s, a, 0);
     launch(k_pcg_update_xr, redBlocks, RED_THREADS, 0, s, a);
     launch(k_pcg_true_residual, redBlocks, RED_THREADS, 0, s, a);
   }
@@ -577,8 +577,7 @@ struct btd_solver {
     encPcgInit(s, a);
     encVCycle(s, 0);
     launch(k_pcg_dot_rz, redBlocks, RED_THREADS, 0, s, a, 1);
-    launch(k_pcg_update_p, blocksFor(N, 256), 256, 0, s, a, 1);
-    launch(k_pcg_matvec, redBlocks, RED_THREADS, 0, s, a);
+    launch(k_pcg_matvec, redBlocks, RED_THREADS, 0, s, a, 1);
     launch(k_pcg_update_xr, redBlocks, RED_THREADS, 0, s, a);
     launch(k_pcg_true_residual, redBlocks, RED_THREADS, 0, s, a);
     CK(cudaStreamGetCaptureInfo(s, &st, nullptr, &g, &deps, &nDeps));
@@ -603,8 +602,7 @@ struct btd_solver {
     encPcgInit(s, a);
     encVCycle(s, 0);
     launch(k_pcg_dot_rz, redBlocks, RED_THREADS, 0, s, a, 1);
-    launch(k_pcg_update_p, blocksFor(N, 256), 256, 0, s, a, 1);
-    launch(k_pcg_matvec, redBlocks, RED_THREADS, 0, s, a);
+    launch(k_pcg_matvec, redBlocks, RED_THREADS, 0, s, a, 1);
     launch(k_pcg_update_xr, redBlocks, RED_THREADS, 0, s, a);
     launch(k_pcg_true_residual, redBlocks, RED_THREADS, 0, s, a);
     for (;;) {
@@ -973,6 +971,7 @@ int btd_create(const btd_scene* sc, const btd_params* prm, btd_solver** out) {
     s->gripOwner.assign(N, -1);
     s->delta = s->alloc<float4>(N);
     s->p = s->alloc<float4>(N);
+    s->p1 = s->alloc<float4>(N);
     s->Ap = s->alloc<float4>(N);
     s->b0 = s->alloc<float4>(N);
     s->deltaD = s->alloc<double>(3 * (size_t)N);
@@ -1837,7 +1836,7 @@ int btd_profile_stage(btd_solver* s, int32_t which, int32_t reps, int32_t flush,
       CK(cudaEventRecord(e0, s->stream));
       switch (which) {
         case BTD_STAGE_MATVEC:
-          k_pcg_matvec<<<s->redBlocks, RED_THREADS, 0, s->stream>>>(pa);
+          k_pcg_matvec<<<s->redBlocks, RED_THREADS, 0, s->stream>>>(pa, 0);
           break;
         case BTD_STAGE_SMOOTH:
           s->encSmooth(s->stream, 0, false);
@@ -1881,8 +1880,8 @@ int btd_launch_count(btd_solver* s, int32_t substeps, int32_t newton, int32_t pc
     const int64_t lc = s->lcOn() ? 1 : 0;
     int64_t V = s->params.coarse_sweeps * colours(L - 1) + lc;
     for (int k = 0; k + 1 < L; ++k) V += 2 * colours(k) + 3;
-    // per Newton iteration: assembly, PCG prologue (init + V-cycle + 5), line search, apply; the
-    // hierarchy (weights + RAP per coarse level) on the first iteration; V-cycle + 5 per extra PCG pass
+    // per Newton iteration: assembly, PCG prologue (init + V-cycle + 4), line search, apply; the
+    // hierarchy (weights + RAP per coarse level) on the first iteration; V-cycle + 4 per extra PCG pass
     // held grips add their lead once per substep and their terms once per Newton iteration; the
     // assembly and every Galerkin product are followed by their level's line factorisation
     const int64_t grips = s->gripsOn() ? 1 : 0;
@@ -1893,13 +1892,13 @@ int btd_launch_count(btd_solver* s, int32_t substeps, int32_t newton, int32_t pc
     const int64_t rigid = s->pieceCount > 0 ? 1 : 0;
     const int64_t xc = s->xcOn() ? 1 : 0;  // cross-layer contact: terms in one kernel, detection in five
     // the learned correction adds its flags (fine, then one a coarse level) and basis to every solve
-    const int64_t perNewton = 2 + (1 + V + 5) + 1 + 1 + grips + (2 - xc) * contact + 4 * rigid + lc * (L + 1);
+    const int64_t perNewton = 2 + (1 + V + 4) + 1 + 1 + grips + (2 - xc) * contact + 4 * rigid + lc * (L + 1);
     const int64_t hierarchy = 3 * (L - 1);
     const int64_t hierPerSubstep = s->params.lag_coarse ? hierarchy : hierarchy * (newton / std::max(1, substeps));
     const int64_t perSubstep = 2 + 1 + 5 + s->nLayers + 4 + grips + (7 - 2 * xc) * contact + 2 * rigid;
     // each optional (gated) Newton iteration slot adds its gate kernel, run or not
     const int64_t gates = s->gatedBound(0, 0) - s->unconditional(0);
-    *out = (int64_t)substeps * (perSubstep + hierPerSubstep + gates) + (int64_t)newton * perNewton + (int64_t)(pcg - newton) * (V + 5);
+    *out = (int64_t)substeps * (perSubstep + hierPerSubstep + gates) + (int64_t)newton * perNewton + (int64_t)(pcg - newton) * (V + 4);
   });
 }
 
