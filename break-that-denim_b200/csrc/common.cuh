@@ -271,11 +271,12 @@ __device__ __forceinline__ float3 m3Vec(const M3& x, float3 v) {
   return make_float3(x.a[0] * v.x + x.a[1] * v.y + x.a[2] * v.z, x.a[3] * v.x + x.a[4] * v.y + x.a[5] * v.z,
                      x.a[6] * v.x + x.a[7] * v.y + x.a[8] * v.z);
 }
-// Inverse of a pivot block shifted by 2e-6 of its largest diagonal entry, with the diagonal fallback
-// for a non-finite result (pivotInverse, common.wgsl:140-150; PIVOT_SHIFT, newtonMultigrid.ts:414).
+// Inverse of a pivot block, with the diagonal fallback for a non-finite result (pivotInverse,
+// common.wgsl:140-150). The reference's shift of the pivots (PIVOT_SHIFT, newtonMultigrid.ts:414) is in the
+// line's rows (lineShift).
 __device__ __forceinline__ M3 pivotInverse(const M3& m) {
   float s = fmaxf(fmaxf(fabsf(m.a[0]), fabsf(m.a[4])), fabsf(m.a[8]));
-  float e = 2e-6f * s + 1e-30f;
+  float e = 1e-30f;
   float a00 = m.a[0] + e, a01 = m.a[1], a02 = m.a[2];
   float a10 = m.a[3], a11 = m.a[4] + e, a12 = m.a[5];
   float a20 = m.a[6], a21 = m.a[7], a22 = m.a[8] + e;

@@ -1,5 +1,8 @@
 // Yarn-line smoother: every line of one colour solved exactly as a block-tridiagonal system
-// (smoothLines + solvePenta, newtonMultigrid.ts:659-733 / 435-473; smooth.wgsl:49-233).
+// (smoothLines + solvePenta, newtonMultigrid.ts:659-733 / 435-473; smooth.wgsl:49-233). Families whose
+// lines are all up to 131 nodes are swept by the kernels of k_line.cuh, which hold a line's coefficients in
+// registers; the two kernels here take the longer lines, whose coefficients fill the shared memory (held in
+// registers, 192 KB a line of 256 nodes, a colour of a 256 x 256 lattice took 5.2 us and takes 4.2 here).
 //
 // The line matrices depend on the operator only, which stays fixed over every PCG iteration of a
 // Newton iteration, so the solve is split in two kernels:
@@ -22,7 +25,7 @@
 // coupling copies (contiguous along the line whatever the family, so every 32-byte sector fetched is
 // used) and five columns of unknowns - the line itself and two lines either side - from which every
 // stencil neighbour is read. Lines of one colour are three apart and never read each other's
-// unknowns (Jacobi within a colour). Every pivot is regularised by pivotInverse. The lower block of
+// unknowns (Jacobi within a colour). Every row is regularised by lineShift. The lower block of
 // row k is the +1 block of row k - 1 (symmetric), as solvePenta takes it.
 //
 // Factor region of a line (float4 units, from the line's base):
@@ -260,6 +263,28 @@ struct Chunks {
   }
 };
 
+// The shift that the reference's solve adds to row k of a line: 2e-6 of its pivot's largest diagonal entry
+// (PIVOT_SHIFT). On a line's softest modes (inertia against spans 1e5 times stiffer) the shifts are of the
+// size of the matrix itself, so they have to be those of the reference's elimination along the line and not of
+// the partition's own pivots, which start every chunk anew: with those a sweep was 5e-4 from the FP64 oracle's,
+// with these it is 2e-5. The pivot's diagonal is followed entry by entry, s_k = B_k - A_k^2 / s_{k-1}, over the
+// LINE_BACK nodes before k; B(q, d) and A(q, d) are diagonal entry d of row q and of the block between q and q + 1.
+constexpr int LINE_BACK = 64;
+template <class GetB, class GetA>
+__device__ __forceinline__ float lineShift(GetB B, GetA A, int k) {
+  const int q0 = max(0, k - LINE_BACK);
+  float s[3] = {B(q0, 0), B(q0, 1), B(q0, 2)};
+#pragma unroll 8
+  for (int q = q0 + 1; q <= k; ++q) {
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const float b = B(q, d), a = A(q - 1, d);
+      s[d] = fmaxf(b - __fdividef(a * a, s[d]), 1e-3f * b);
+    }
+  }
+  return 2e-6f * fmaxf(fmaxf(s[0], s[1]), s[2]);
+}
+
 // ------------------------------------------------------------------------------------------ factor
 
 // Line row of node (i, j) from its staged row planes: B = D + maj I, C the +1 block (zero at the
@@ -339,6 +364,21 @@ __global__ void __launch_bounds__(SM_THREADS) k_line_factor(DLevel L, const int4
     stS(sB + 2 * k, Bk);
     stS(sC + 2 * k, Ck);
     sF[2 * NP + ch.idx(k)] = make_float4(0.f, maj, L.fixed[n] != 0u ? 1.f : 0.f, 0.f);
+  }
+  __syncthreads();
+  // ---- the rows' shifts, found before any is added
+  auto diagonal = [](const float4* p, int d) { return d == 0 ? p[0].x : d == 1 ? p[0].w : p[1].y; };
+  float shift[(SM_MAX_LINE + SM_THREADS - 1) / SM_THREADS];
+#pragma unroll
+  for (int q = 0; q < (SM_MAX_LINE + SM_THREADS - 1) / SM_THREADS; ++q) {
+    const int k = tid + q * SM_THREADS;
+    shift[q] = k < len ? lineShift([&](int r, int d) { return diagonal(sB + 2 * r, d); }, [&](int r, int d) { return diagonal(sC + 2 * r, d); }, k) : 0.f;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < (SM_MAX_LINE + SM_THREADS - 1) / SM_THREADS; ++q) {
+    const int k = tid + q * SM_THREADS;
+    if (k < len) stS(sB + 2 * k, ldS(sB + 2 * k) + symId(shift[q]));
   }
   __syncthreads();
 

@@ -25,6 +25,7 @@
 #include "k_contact.cuh"
 #include "k_grip.cuh"
 #include "k_learned.cuh"
+#include "k_line.cuh"
 #include "k_xcontact.cuh"
 #include "k_history.cuh"
 #include "k_mg.cuh"
@@ -56,6 +57,9 @@ struct Level {
   std::vector<int4> lines;  // (start, stride, length, family) grouped by colour
   int colourStart[7] = {0, 0, 0, 0, 0, 0, 0};
   int maxLine = 0;
+  int famLine[2] = {0, 0};  // longest line of each family
+  // the families whose lines the compact sweep takes (k_line.cuh); the others go through k_smooth
+  bool compact(int fam) const { return !fine && famLine[fam] <= CUT_LINE; }
   DLevelLayer* dLayers = nullptr;
   uint2* dCoord = nullptr;
   int4* dLines = nullptr;
@@ -97,24 +101,29 @@ static void buildLines(Level& L) {
     const int tag = (int)(l << 1);
     for (int i = 0; i < ly.nx; ++i) byColour[i % 3].push_back(make_int4(ly.offset + i, ly.nx, ly.ny, 1 | tag));
     for (int j = 0; j < ly.ny; ++j) byColour[3 + j % 3].push_back(make_int4(ly.offset + j * ly.nx, 1, ly.nx, 0 | tag));
-    L.maxLine = std::max(L.maxLine, std::max(ly.nx, ly.ny));
+    L.famLine[0] = std::max(L.famLine[0], ly.nx);
+    L.famLine[1] = std::max(L.famLine[1], ly.ny);
   }
+  L.maxLine = std::max(L.famLine[0], L.famLine[1]);
   L.lines.clear();
   for (int c = 0; c < 6; ++c) {
     L.colourStart[c] = (int)L.lines.size();
     L.lines.insert(L.lines.end(), byColour[c].begin(), byColour[c].end());
   }
   L.colourStart[6] = (int)L.lines.size();
-  auto regionF4 = [&](int len) { return L.fine ? lineFactorF4<FineRows>(len) : lineFactorF4<CoarseRows>(len); };
+  auto regionF4 = [&](int len, int fam) {
+    if (L.compact(fam)) return L.fine ? cutF4<FineRows>(len) : cutF4<CoarseRows>(len);
+    return L.fine ? lineFactorF4<FineRows>(len) : lineFactorF4<CoarseRows>(len);
+  };
   L.facBase.clear();
   size_t off = 0;
   for (const int4& ln : L.lines) {
     L.facBase.push_back((int)off);
-    off += regionF4(ln.z);
+    off += regionF4(ln.z, ln.w & 1);
   }
   L.facF4 = off;
   L.tile = L.fine ? smoothTile<FineRows>(L.maxLine) : smoothTile<CoarseRows>(L.maxLine);
-  L.threads = sweepThreads(L.maxLine);
+  L.threads = L.compact(0) && L.compact(1) ? std::min(SM_SWEEP_THREADS, cutThreads(L.maxLine)) : sweepThreads(L.maxLine);
   for (int c = 0; c < 6; ++c) {
     LineGeom& g = L.geom[c];
     g = LineGeom{};
@@ -129,10 +138,15 @@ static void buildLines(Level& L) {
     g.stride = fam == 1 ? ly.nx : 1;
     g.len = fam == 1 ? ly.ny : ly.nx;
     g.base0 = L.facBase[g.first];
-    g.baseStep = regionF4(g.len);
+    g.baseStep = regionF4(g.len, fam);
     g.across0 = c3;
-    const Chunks ch(g.len);
-    g.P = ch.P, g.chunkBase = ch.base, g.chunkExtra = ch.extra, g.S = ch.S;
+    if (L.compact(fam)) {
+      const Cut cut(g.len);
+      g.P = cut.P, g.chunkBase = cut.base, g.chunkExtra = cut.extra;
+    } else {
+      const Chunks ch(g.len);
+      g.P = ch.P, g.chunkBase = ch.base, g.chunkExtra = ch.extra, g.S = ch.S;
+    }
     bool same = true;
     for (int b = 0; b < L.colourStart[c + 1] - g.first; ++b) {
       const int4 ln = L.lines[g.first + b];
@@ -470,14 +484,28 @@ struct btd_solver {
     }
   }
 
-  // Line factors of level k, every line in one launch (after its operator changed).
+  // Line factors of level k, every line of a family in one launch (after its operator changed).
   void encFactor(cudaStream_t s, int k) {
     Level& L = levels[k];
-    const int count = (int)L.lines.size();
-    if (L.fine)
-      k_line_factor<FineRows><<<count, SM_THREADS, factorSmemBytes<FineRows>(L.maxLine), s>>>(L.dev(), L.dLines, L.dFacBase, L.fac);
+    const int split = L.colourStart[3], all = (int)L.lines.size();  // v-lines, then u-lines
+    if (L.compact(0) && L.compact(1)) {
+      encFactorLines(s, L, 0, all, L.maxLine, true);
+    } else {
+      encFactorLines(s, L, 0, split, L.famLine[1], L.compact(1));
+      encFactorLines(s, L, split, all - split, L.famLine[0], L.compact(0));
+    }
+  }
+  void encFactorLines(cudaStream_t s, const Level& L, int first, int count, int len, bool compact) {
+    const int4* lines = L.dLines + first;
+    const int* base = L.dFacBase + first;
+    if (compact && L.fine)
+      k_line_compact<FineRows><<<count, std::min(CUT_FACTOR_THREADS, cutThreads(len)), cutFactorSmem(len), s>>>(L.dev(), lines, base, L.fac);
+    else if (compact)
+      k_line_compact<CoarseRows><<<count, std::min(CUT_FACTOR_THREADS, cutThreads(len)), cutFactorSmem(len), s>>>(L.dev(), lines, base, L.fac);
+    else if (L.fine)
+      k_line_factor<FineRows><<<count, SM_THREADS, factorSmemBytes<FineRows>(len), s>>>(L.dev(), lines, base, L.fac);
     else
-      k_line_factor<CoarseRows><<<count, SM_THREADS, factorSmemBytes<CoarseRows>(L.maxLine), s>>>(L.dev(), L.dLines, L.dFacBase, L.fac);
+      k_line_factor<CoarseRows><<<count, SM_THREADS, factorSmemBytes<CoarseRows>(len), s>>>(L.dev(), lines, base, L.fac);
   }
 
   // One sweep of level k: the six colours, v-lines first (reversed for the post-smoother).
@@ -507,7 +535,9 @@ struct btd_solver {
       const int count = L.colourStart[c + 1] - L.colourStart[c];
       if (count == 0) continue;
       const LineGeom& g = L.geom[c];
-      if (L.fine) {
+      if (L.compact(c < 3 ? 1 : 0)) {
+        encSweep(s, L, d, c);
+      } else if (L.fine) {
         if (c < 3)
           launch(k_smooth<FineRows, 1>, count, L.threads, smem, s, d, g, (const int4*)L.dLines, (const int*)L.dFacBase, (const float4*)L.fac, L.tile, dCounters + CNT_ERROR);
         else
@@ -519,6 +549,21 @@ struct btd_solver {
           launch(k_smooth<CoarseRows, 0>, count, L.threads, smem, s, d, g, (const int4*)L.dLines, (const int*)L.dFacBase, (const float4*)L.fac, L.tile, dCounters + CNT_ERROR);
       }
     }
+  }
+
+  // One colour of a compact family.
+  void encSweep(cudaStream_t s, const Level& L, const DLevel& d, int c) {
+    const int count = L.colourStart[c + 1] - L.colourStart[c], len = L.famLine[c < 3 ? 1 : 0], nt = cutThreads(len);
+    auto go = [&](auto k) {
+      launch(k, count, nt, cutSweepSmem(len), s, d, L.geom[c], (const int4*)L.dLines, (const int*)L.dFacBase, (const float4*)L.fac);
+    };
+    auto rows = [&](auto v, auto u) { c < 3 ? go(v) : go(u); };
+    if (nt <= 160)
+      L.fine ? rows(k_sweep<FineRows, 1, 160, 3>, k_sweep<FineRows, 0, 160, 3>) : rows(k_sweep<CoarseRows, 1, 160, 3>, k_sweep<CoarseRows, 0, 160, 3>);
+    else if (nt <= 288)
+      L.fine ? rows(k_sweep<FineRows, 1, 288, 2>, k_sweep<FineRows, 0, 288, 2>) : rows(k_sweep<CoarseRows, 1, 288, 2>, k_sweep<CoarseRows, 0, 288, 2>);
+    else
+      L.fine ? rows(k_sweep<FineRows, 1, 544, 1>, k_sweep<FineRows, 0, 544, 1>) : rows(k_sweep<CoarseRows, 1, 544, 1>, k_sweep<CoarseRows, 0, 544, 1>);
   }
 
   // encodeVCycle (solver.ts:584-598): X of level k = V(B) with X zero on entry.
@@ -1059,7 +1104,7 @@ int btd_create(const btd_scene* sc, const btd_params* prm, btd_solver** out) {
       const size_t smem = L.fine ? smoothSmemBytes<FineRows>(L.maxLine, L.tile) : smoothSmemBytes<CoarseRows>(L.maxLine, L.tile);
       const size_t fsmem = L.fine ? factorSmemBytes<FineRows>(L.maxLine) : factorSmemBytes<CoarseRows>(L.maxLine);
       // (227 KB of opt-in shared memory a block, less the kernels' few bytes of static shared memory)
-      if (L.maxLine > SM_MAX_LINE || smem > 226 * 1024 || fsmem > 226 * 1024)
+      if (!(L.compact(0) && L.compact(1)) && (L.maxLine > SM_MAX_LINE || smem > 226 * 1024 || fsmem > 226 * 1024))
         throw std::invalid_argument("yarn lines of " + std::to_string(L.maxLine) + " nodes exceed the smoother's shared memory");
     }
 
@@ -1085,6 +1130,8 @@ int btd_create(const btd_scene* sc, const btd_params* prm, btd_solver** out) {
         set((const void*)k_smooth<CoarseRows, 1>);
         set((const void*)k_line_factor<FineRows>);
         set((const void*)k_line_factor<CoarseRows>);
+        set((const void*)k_line_compact<FineRows>);
+        set((const void*)k_line_compact<CoarseRows>);
         smemErr = e;
       });
       CK(smemErr);
@@ -1789,12 +1836,14 @@ int btd_autotune(btd_solver* s, int32_t reps, int32_t* threads_out, int32_t* til
     CK(cudaEventCreate(&e1));
     for (size_t k = 0; k < s->levels.size(); ++k) {
       Level& L = s->levels[k];
+      const bool fixedShape = L.compact(0) && L.compact(1);  // four threads a node (k_sweep): timed, nothing to choose
       std::vector<int> tiles{L.tile};
-      if (L.maxLine > 128 && L.tile != 128) tiles.push_back(128);
+      if (!fixedShape && L.maxLine > 128 && L.tile != 128) tiles.push_back(128);
       int bestT = L.threads, bestTile = L.tile;
       float best = 1e30f;
       for (int tile : tiles)
         for (int T = 64; T <= SM_SWEEP_THREADS; T += 32) {
+          if (fixedShape) T = L.threads;
           L.tile = tile;
           L.threads = T;
           s->encSmooth(s->stream, (int)k, false);  // untimed: first touch
@@ -1806,6 +1855,7 @@ int btd_autotune(btd_solver* s, int32_t reps, int32_t* threads_out, int32_t* til
           CK(cudaEventElapsedTime(&t, e0, e1));
           t /= reps;
           if (t < best) best = t, bestT = T, bestTile = tile;
+          if (fixedShape) break;
         }
       L.threads = bestT;
       L.tile = bestTile;
