@@ -155,13 +155,16 @@ __device__ __forceinline__ bool mbarTryWait(uint64_t* bar, unsigned parity) {
 constexpr int MBAR_TRIES = 1 << 20;
 constexpr uint32_t ERR_COPY_TIMEOUT = 1u;
 __device__ int g_mbarFirstTries = MBAR_TRIES;
-__device__ __forceinline__ void mbarWaitBounded(uint64_t* bar, unsigned parity, uint32_t* err) {
-  const int first = g_mbarFirstTries;
+template <class Try>
+__device__ __forceinline__ void mbarWaitBounded(uint64_t* bar, unsigned parity, uint32_t* err, Try tryWait, int first) {
   for (int i = 0; i < first; ++i)
-    if (mbarTryWait(bar, parity)) return;
+    if (tryWait(bar, parity)) return;
   if (err) atomicOr(err, ERR_COPY_TIMEOUT);
   for (int i = 0; i < MBAR_TRIES; ++i)
-    if (mbarTryWait(bar, parity)) return;
+    if (tryWait(bar, parity)) return;
+}
+__device__ __forceinline__ void mbarWaitBounded(uint64_t* bar, unsigned parity, uint32_t* err) {
+  mbarWaitBounded(bar, parity, err, [](uint64_t* b, unsigned p) { return mbarTryWait(b, p); }, g_mbarFirstTries);
 }
 
 // 3x3 blocks padded to 12 floats (three float4, strided by `s` float4).

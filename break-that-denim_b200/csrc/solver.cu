@@ -32,6 +32,7 @@
 #include "k_pcg.cuh"
 #include "k_rigid.cuh"
 #include "k_smooth.cuh"
+#include "k_tail.cuh"
 #include "k_step.cuh"
 
 namespace btd {
@@ -275,6 +276,15 @@ struct btd_solver {
   std::map<int, cudaGraphExec_t> substepExec;
   cudaGraphExec_t pcgExec = nullptr;
   bool useGraphs = true;
+  // While a substep of a batch is captured: its coarse levels keep their launches, as a cluster needs sixteen
+  // SMs of one GPC at once that the other patches' lines are on. The arithmetic is the same bit for bit.
+  bool batched = false;
+  // the levels from here down run as one cluster launch (k_tail; -1: none)
+  int tailFrom = -1;
+  TailVisit* dTailVisits = nullptr;
+  int* dTailOps = nullptr;
+  TailArgs tailArgs{};
+  int tailOps = 0, tailVisits = 0, tailMidOp = 0, tailMidVisit = 0;  // all, and those before the learned correction
   bool batchGrips = false;  // grips held when a batch graph holding this solver was captured
   void* flushBuf = nullptr;  // profiling only: rewritten to evict L2 between timed launches
 
@@ -566,9 +576,132 @@ struct btd_solver {
       L.fine ? rows(k_sweep<FineRows, 1, 544, 1>, k_sweep<FineRows, 0, 544, 1>) : rows(k_sweep<CoarseRows, 1, 544, 1>, k_sweep<CoarseRows, 0, 544, 1>);
   }
 
+  // The V-cycle below (and of) level tailFrom, ops [op0, op1) and colours [v0, v1) of it.
+  void encTail(cudaStream_t s, int op0, int op1, int v0, int v1, bool load) {
+    TailArgs a = tailArgs;
+    a.op0 = op0, a.op1 = op1, a.visit0 = v0, a.visits1 = v1;
+    a.load = load ? 1 : 0;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = TAIL_CTAS;
+    cfg.blockDim = TAIL_THREADS;
+    cfg.dynamicSmemBytes = 16 * (size_t)a.f4;
+    cfg.stream = s;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = TAIL_CTAS, at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = params.overlap_launches ? 2 : 1;
+    if (levels[tailFrom].fine)
+      CK(cudaLaunchKernelEx(&cfg, k_tail<FineRows>, a));
+    else
+      CK(cudaLaunchKernelEx(&cfg, k_tail<CoarseRows>, a));
+  }
+
+  // Sets the tail up: the levels whose colours have at most TAIL_CTAS lines, from the coarsest up (coarse
+  // rows; a lattice with a single level is swept whole), when the device can hold the cluster.
+  void buildTail() {
+    const int last = (int)levels.size() - 1;
+    auto fits = [&](const Level& L) {
+      return L.layers.size() == 1 && L.layers[0].nx <= TAIL_SIDE && L.layers[0].ny <= TAIL_SIDE;
+    };
+    int from = last + 1;
+    while (from > 0 && last + 1 - from < TAIL_LEVELS && fits(levels[from - 1]) && !levels[from - 1].fine) --from;
+    const int n = last + 1 - from;
+    if (n == 0) return;
+    std::vector<TailVisit> visits;
+    std::vector<int> ops;
+    TailArgs& a = tailArgs;
+    a.levels = n;
+    int at = 0;
+    for (int l = 0; l < n; ++l) {
+      const Level& L = levels[from + l];
+      a.lev[l].d = L.dev();
+      a.fac[l] = L.fac;
+      a.lev[l].W = L.layers[0].nx + 4;
+      a.lev[l].x0 = at + 2 * a.lev[l].W + 2;
+      at += a.lev[l].W * (L.layers[0].ny + 4);
+      a.lev[l].b0 = l == 0 ? -1 : at;
+      if (l > 0) at += L.N;
+    }
+    a.rAt = at, at += levels[from].N;
+    a.tokenAt = at, at += 1;
+    a.scratchAt = at, at += cutScratchF4(TAIL_SIDE);
+    a.f4 = at;
+    auto sweep = [&](int l, bool reverse) {
+      const Level& L = levels[from + l];
+      for (int q = 0; q < 6; ++q) {
+        const int c = reverse ? 5 - q : q, count = L.colourStart[c + 1] - L.colourStart[c], fam = c < 3 ? 1 : 0;
+        if (count == 0) continue;
+        int nodes = 0;
+        for (int b = 0; b < count; ++b) nodes += L.lines[L.colourStart[c] + b].z;
+        for (int r = 0; r < TAIL_CTAS; ++r) {
+          TailVisit v{};
+          v.level = l;
+          v.bytes = tailBytes(nodes, count);
+          if (r < count) {
+            const int4 ln = L.lines[L.colourStart[c] + r];
+            const int W = a.lev[l].W, i = ln.x % L.layers[0].nx, j = ln.x / L.layers[0].nx;
+            const Cut cut(ln.z);
+            v.len = ln.z, v.fac = L.facBase[L.colourStart[c] + r], v.n0 = ln.x, v.st = ln.y;
+            v.x0 = a.lev[l].x0 + j * W + i, v.along = fam == 1 ? W : 1, v.across = fam == 1 ? 1 : W;
+            v.P = cut.P, v.base = cut.base, v.extra = cut.extra;
+          }
+          visits.push_back(v);
+        }
+        ops.push_back(TAIL_PASS), ops.push_back(l);
+      }
+    };
+    for (int l = 0; l + 1 < n; ++l) {
+      sweep(l, false);
+      ops.push_back(TAIL_RESTRICT), ops.push_back(l);
+    }
+    for (int sw = 0; sw < params.coarse_sweeps; ++sw) {
+      if (sw == params.coarse_sweeps / 2) tailMidOp = (int)ops.size() / 2, tailMidVisit = (int)visits.size() / TAIL_CTAS;
+      sweep(n - 1, (sw & 1) == 1);
+    }
+    for (int l = n - 2; l >= 0; --l) {
+      ops.push_back(TAIL_PROLONG), ops.push_back(l);
+      sweep(l, true);
+    }
+    tailOps = (int)ops.size() / 2, tailVisits = (int)visits.size() / TAIL_CTAS;
+    if (tailVisits > TAIL_VISITS || 16 * (size_t)a.f4 > 200 * 1024) return;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = TAIL_CTAS, cfg.blockDim = TAIL_THREADS, cfg.dynamicSmemBytes = 16 * (size_t)a.f4;
+    cudaLaunchAttribute cl;
+    cl.id = cudaLaunchAttributeClusterDimension;
+    cl.val.clusterDim.x = TAIL_CTAS, cl.val.clusterDim.y = cl.val.clusterDim.z = 1;
+    cfg.attrs = &cl, cfg.numAttrs = 1;
+    int clusters = 0;
+    const cudaError_t e = levels[from].fine ? cudaOccupancyMaxActiveClusters(&clusters, k_tail<FineRows>, &cfg)
+                                            : cudaOccupancyMaxActiveClusters(&clusters, k_tail<CoarseRows>, &cfg);
+    if (e != cudaSuccess) cudaGetLastError();
+    if (e != cudaSuccess || clusters < 1) return;
+    dTailVisits = alloc<TailVisit>(visits.size());
+    dTailOps = alloc<int>(ops.size());
+    CK(cudaMemcpyAsync(dTailVisits, visits.data(), sizeof(TailVisit) * visits.size(), cudaMemcpyHostToDevice, stream));
+    CK(cudaMemcpyAsync(dTailOps, ops.data(), sizeof(int) * ops.size(), cudaMemcpyHostToDevice, stream));
+    CK(cudaStreamSynchronize(stream));
+    a.visits = dTailVisits;
+    a.ops = dTailOps;
+    a.err = dCounters + CNT_ERROR;
+    tailFrom = from;
+  }
+
   // encodeVCycle (solver.ts:584-598): X of level k = V(B) with X zero on entry.
   void encVCycle(cudaStream_t s, int k) {
     int last = (int)levels.size() - 1;
+    if (k == tailFrom && !batched) {
+      if (lcOn()) {
+        encTail(s, 0, tailMidOp, 0, tailMidVisit, false);
+        launch(k_lc_correct, 1, LC_THREADS, 0, s, levels[last].dev(), lcArgs());
+        encTail(s, tailMidOp, tailOps, tailMidVisit, tailVisits, true);
+      } else {
+        encTail(s, 0, tailOps, 0, tailVisits, false);
+      }
+      return;
+    }
     if (k == last) {
       if (lcOn()) {
         // the learned coarse space half-way through the coarsest sweeps, which mirror around it
@@ -798,12 +931,20 @@ struct btd_solver {
     return std::min(MAX_NEWTON, std::max(std::max(params.newton_max, unconditional(minIterations)), maxIterations));
   }
 
-  cudaGraphExec_t substepGraph(int iters, int itersMax) {
+  cudaGraphExec_t substepGraph(int iters, int itersMax, bool inBatch = false) {
     const bool grips = gripsOn();
-    const int key = (iters * (MAX_NEWTON + 1) + itersMax) * 2 + (grips ? 1 : 0);
+    const int key = ((iters * (MAX_NEWTON + 1) + itersMax) * 2 + (grips ? 1 : 0)) * 2 + (inBatch ? 1 : 0);
     auto it = substepExec.find(key);
     if (it != substepExec.end()) return it->second;
-    cudaGraphExec_t ex = capture([&](cudaStream_t s) { encSubstep(s, iters, itersMax, grips); });
+    batched = inBatch;
+    cudaGraphExec_t ex = nullptr;
+    try {
+      ex = capture([&](cudaStream_t s) { encSubstep(s, iters, itersMax, grips); });
+    } catch (...) {
+      batched = false;
+      throw;
+    }
+    batched = false;
     substepExec[key] = ex;
     return ex;
   }
@@ -1130,12 +1271,20 @@ int btd_create(const btd_scene* sc, const btd_params* prm, btd_solver** out) {
         set((const void*)k_smooth<CoarseRows, 1>);
         set((const void*)k_line_factor<FineRows>);
         set((const void*)k_line_factor<CoarseRows>);
+        auto cluster = [&](const void* f) {
+          set(f);
+          if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        };
+        cluster((const void*)k_tail<FineRows>);
+        cluster((const void*)k_tail<CoarseRows>);
         set((const void*)k_line_compact<FineRows>);
         set((const void*)k_line_compact<CoarseRows>);
         smemErr = e;
       });
       CK(smemErr);
     }
+
+    s->buildTail();
 
     // ---- parameters
     SimParams& P = s->hostP;
@@ -1208,7 +1357,7 @@ int btd_batch_substeps(btd_solver* const* solvers, int32_t count, int32_t subste
     for (int b = 0; b < count; ++b) {
       btd_solver* s = solvers[b];
       checkSolver(s);
-      if (s->useGraphs) graphs[b] = s->substepGraph(s->unconditional(0), s->gatedBound(0, 0));
+      if (s->useGraphs) graphs[b] = s->substepGraph(s->unconditional(0), s->gatedBound(0, 0), count > 1);
     }
     // round robin: every patch's next substep is queued before any patch's one after, so all
     // streams have work from the start
@@ -1255,7 +1404,14 @@ struct btd_batch {
       for (size_t b = 0; b < solvers.size(); ++b) {
         btd_solver* s = solvers[b];
         CK(cudaStreamWaitEvent(s->stream, fork, 0));
-        s->encSubstep(s->stream, s->unconditional(0), s->gatedBound(0, 0), s->gripsOn());
+        s->batched = true;
+        try {
+          s->encSubstep(s->stream, s->unconditional(0), s->gatedBound(0, 0), s->gripsOn());
+        } catch (...) {
+          s->batched = false;
+          throw;
+        }
+        s->batched = false;
         CK(cudaEventRecord(done[b], s->stream));
         CK(cudaStreamWaitEvent(stream, done[b], 0));
       }
@@ -1928,8 +2084,9 @@ int btd_launch_count(btd_solver* s, int32_t substeps, int32_t newton, int32_t pc
     };
     const int L = (int)s->levels.size();
     const int64_t lc = s->lcOn() ? 1 : 0;
-    int64_t V = s->params.coarse_sweeps * colours(L - 1) + lc;
-    for (int k = 0; k + 1 < L; ++k) V += 2 * colours(k) + 3;
+    const int tail = s->tailFrom >= 0 ? s->tailFrom : L - 1;  // from here down one launch, two around the learned correction
+    int64_t V = (s->tailFrom >= 0 ? 1 + lc : s->params.coarse_sweeps * colours(L - 1)) + lc;
+    for (int k = 0; k < tail; ++k) V += 2 * colours(k) + 3;
     // per Newton iteration: assembly, PCG prologue (init + V-cycle + 4), line search, apply; the
     // hierarchy (weights + RAP per coarse level) on the first iteration; V-cycle + 4 per extra PCG pass
     // held grips add their lead once per substep and their terms once per Newton iteration; the
