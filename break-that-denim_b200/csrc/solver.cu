@@ -60,7 +60,7 @@ struct Level {
   int maxLine = 0;
   int famLine[2] = {0, 0};  // longest line of each family
   // the families whose lines the compact sweep takes (k_line.cuh); the others go through k_smooth
-  bool compact(int fam) const { return !fine && famLine[fam] <= CUT_LINE; }
+  bool compact(int fam) const { return famLine[fam] <= CUT_LINE; }
   DLevelLayer* dLayers = nullptr;
   uint2* dCoord = nullptr;
   int4* dLines = nullptr;
@@ -607,7 +607,7 @@ struct btd_solver {
       return L.layers.size() == 1 && L.layers[0].nx <= TAIL_SIDE && L.layers[0].ny <= TAIL_SIDE;
     };
     int from = last + 1;
-    while (from > 0 && last + 1 - from < TAIL_LEVELS && fits(levels[from - 1]) && !levels[from - 1].fine) --from;
+    while (from > 0 && last + 1 - from < TAIL_LEVELS && fits(levels[from - 1]) && (!levels[from - 1].fine || last == 0)) --from;
     const int n = last + 1 - from;
     if (n == 0) return;
     std::vector<TailVisit> visits;
