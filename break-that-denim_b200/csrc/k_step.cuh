@@ -312,11 +312,35 @@ __device__ __forceinline__ SymD springBlockD(const StepArgs& A, int a, int b, fl
 // Normal stiffness of an active contact bound relative to the node's own diagonal (assemble.wgsl:142).
 constexpr float ACTIVE_BOUND = 100.f;
 
+// The right-hand side of node n in FP64: its FP32 part of the terms (the drag block) as k_assemble forms it.
+__device__ __forceinline__ void assembleRhs(const StepArgs& A, int n, float4* __restrict__ rhs) {
+  if (A.pinned[n]) {
+    rhs[n] = make_float4(0, 0, 0, 0);
+    return;
+  }
+  const SimParams P = *A.P;
+  const NodeStatic st = A.nodes[n];
+  const int i = st.ij & 0xFFFF, j = st.ij >> 16;
+  const DLayer& L = A.layers[st.layer];
+  const Dv gd = gradientD(A, n, P, st, L, i, j, airDragBlock(A, n, L, i, j, P.h));
+  rhs[n] = make_float4((float)-gd.x, (float)-gd.y, (float)-gd.z, 0.f);
+}
+
+// The rows of the projected Newton system, a thread a node, and its right-hand side: the FP64 gradient by the
+// second half of the grid (a thread a node too), so that a lattice that does not fill the GPU's SMs pays for the
+// longer of the two chains and not for their sum.
 __global__ void __launch_bounds__(128) k_assemble(StepArgs A, float4* __restrict__ op, float4* __restrict__ rhs,
                                                   double2* __restrict__ op64) {
+  const int half = gridDim.x / 2;
+  if ((int)blockIdx.x >= half) {
+    const int m = (blockIdx.x - half) * blockDim.x + threadIdx.x;
+    if (m < A.N && A.P->gradFp64) assembleRhs(A, m, rhs);
+    return;
+  }
   int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= A.N) return;
   const int N = A.N;
+  const bool fp32Rhs = A.P->gradFp64 == 0;
   float row[60];
 #pragma unroll
   for (int q = 0; q < 60; ++q) row[q] = 0.f;
@@ -327,7 +351,7 @@ __global__ void __launch_bounds__(128) k_assemble(StepArgs A, float4* __restrict
     if (op64)
       for (int q = 0; q < FINE64_PLANES; ++q)  // the identity block: values 0, 3 and 5
         op64[(size_t)q * N + n] = make_double2(q == 0 ? 1.0 : 0.0, q == 1 || q == 2 ? 1.0 : 0.0);
-    rhs[n] = make_float4(0, 0, 0, 0);
+    if (fp32Rhs) rhs[n] = make_float4(0, 0, 0, 0);
     return;
   }
   const SimParams P = *A.P;
@@ -505,12 +529,7 @@ __global__ void __launch_bounds__(128) k_assemble(StepArgs A, float4* __restrict
   row[54] = C2[0], row[55] = C2[1], row[56] = C2[2], row[57] = C2[3];
 #pragma unroll
   for (int p = 0; p < FINE_PLANES; ++p) op[(size_t)p * N + n] = make_float4(row[4 * p], row[4 * p + 1], row[4 * p + 2], row[4 * p + 3]);
-  if (P.gradFp64) {
-    const Dv gd = gradientD(A, n, P, st, L, i, j, Dd);
-    rhs[n] = make_float4((float)-gd.x, (float)-gd.y, (float)-gd.z, 0.f);
-    return;
-  }
-  rhs[n] = make_float4(-g.x, -g.y, -g.z, 0.f);
+  if (fp32Rhs) rhs[n] = make_float4(-g.x, -g.y, -g.z, 0.f);
 }
 
 // A half-space bound: the step may move against m.xyz by at most m.w (step.wgsl:62-65).

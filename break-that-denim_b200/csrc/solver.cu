@@ -476,7 +476,7 @@ struct btd_solver {
   }
 
   void encAssemble(cudaStream_t s, bool coarse) {
-    k_assemble<<<blocksFor(N, 128), 128, 0, s>>>(stepArgs(), levels[0].op, levels[0].B, opFp64 ? op64 : nullptr);
+    k_assemble<<<2 * blocksFor(N, 128), 128, 0, s>>>(stepArgs(), levels[0].op, levels[0].B, opFp64 ? op64 : nullptr);
     if (pieceCount > 0) {  // the pieces' rigid frames at this iterate (encodeAssemble, solver.ts:615-616)
       k_rigid_rotation<<<blocksFor(N, 128), 128, 0, s>>>(stepArgs(), rigidArgs());
       k_rigid_frame<<<pieceCount, RIGID_THREADS, 0, s>>>(stepArgs(), rigidArgs());
