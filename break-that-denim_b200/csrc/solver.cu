@@ -168,7 +168,8 @@ struct btd_solver {
   btd_params params{};
   SimParams hostP{};
   int N = 0, C = 0, nLayers = 0;
-  int redBlocks = 1;
+  int redBlocks = 1, redPartials = 1;
+  static constexpr int ENERGY_WAVE = 4 * 148;  // most blocks of the line search's four-lane form (37,888 nodes)
   std::vector<void*> allocs;
   // scene copies for resetState
   std::vector<float4> x0;
@@ -829,7 +830,11 @@ struct btd_solver {
       e.red = reduce();
       e.curveW = pieceCount > 0 ? dCurveW : nullptr;
       e.curveR = pieceCount > 0 ? dCurveR : nullptr;
-      k_energy<<<redBlocks, RED_THREADS, 0, s>>>(e);
+      const int blocks = blocksFor(4 * N, RED_THREADS);
+      if (blocks <= ENERGY_WAVE)
+        k_energy<4><<<blocks, RED_THREADS, 0, s>>>(e);
+      else
+        k_energy<1><<<redBlocks, RED_THREADS, 0, s>>>(e);
     } else {
       k_set_alpha<<<1, 1, 0, s>>>(dScal, dCounters, 1.f);
     }
@@ -1122,7 +1127,8 @@ int btd_create(const btd_scene* sc, const btd_params* prm, btd_solver** out) {
     s->dScal = s->alloc<Scalars>(1);
     s->dCounters = s->alloc<uint32_t>(CNT_SIZE);
     s->redBlocks = std::max(1, std::min(blocksFor(N, RED_THREADS), 4 * 148));
-    s->dPartials = s->alloc<double>(8 * (size_t)s->redBlocks);
+    s->redPartials = std::max(s->redBlocks, std::min(blocksFor(4 * N, RED_THREADS), btd_solver::ENERGY_WAVE));
+    s->dPartials = s->alloc<double>(8 * (size_t)s->redPartials);
     s->dTicket = s->alloc<unsigned>(1);
     s->dNodes = s->alloc<NodeStatic>(N);
     s->dLayers = s->alloc<DLayer>(s->hostLayers.size());
