@@ -254,11 +254,39 @@ __device__ __forceinline__ void symVecAddD(const Sym& A, const double* x, double
   y2 += (double)A.xz * x[0] + (double)A.yz * x[1] + (double)A.zz * x[2];
 }
 
-// y += (row n of the fine operator) x, in FP64, from the FP64 rows (null: the fp32 rows, their products
-// summed in FP64); X the type that xAt gives the unknowns in. The row and the thirteen unknowns are all loaded before the first product
-// (a neighbour outside the layer reads the node itself and is left out of the sum), so that they take one
-// round trip to L2 and not one a neighbour (with the direction's update inside, k_pcg_matvec, a PCG iteration of
-// 16 x 16 nodes takes 40 us and took 48).
+// y += (row n of the operator PCG solves with) x, in FP64: the FP64 row when there is one, else the fp32
+// row's products summed in FP64. xAt(m, q) puts node m's x in q and returns false for a node whose x is
+// zero (skipped).
+template <class X, class XAt>
+__device__ __forceinline__ void pcgRowApply(const DLevel& F, const double2* __restrict__ op64, int n, XAt xAt, double& y0, double& y1,
+                                            double& y2) {
+  int i, j, l;
+  nodeAt(F, n, &i, &j, &l);
+  const DLevelLayer L = layerOf(F, l);
+  X q[3];
+  if (xAt(n, q)) {
+    const double x[3] = {(double)q[0], (double)q[1], (double)q[2]};
+    if (op64)
+      symDVecAdd(loadSymD(op64, F.N, n, 0), x, y0, y1, y2);
+    else
+      symVecAddD(FineRows::diag(F.op, F.N, n), x, y0, y1, y2);
+  }
+#pragma unroll
+  for (int k = 0; k < FineRows::NC; ++k) {
+    const int2 off = FineRows::offset(k);
+    const int m = levelNode(L, i + off.x, j + off.y);
+    if (m < 0 || !xAt(m, q)) continue;
+    const double x[3] = {(double)q[0], (double)q[1], (double)q[2]};
+    if (op64)
+      symDVecAdd(fine64Block(op64, F.N, n, k), x, y0, y1, y2);
+    else
+      symVecAddD(FineRows::coupling(F.op, F.N, n, k), x, y0, y1, y2);
+  }
+}
+
+// The same with every load of the row and of its thirteen unknowns issued before the first product (a
+// neighbour outside the layer reads the node itself and is left out of the sum), so that they take one round
+// trip to L2 and not one a neighbour; X is the type that xAt gives the unknowns in.
 template <class X, class XAt>
 __device__ __forceinline__ void pcgRowGather(const DLevel& F, const double2* __restrict__ op64, int n, XAt xAt, double& y0, double& y1,
                                              double& y2) {
@@ -306,10 +334,25 @@ __device__ __forceinline__ void pcgRowGather(const DLevel& F, const double2* __r
   }
 }
 
+// One of the two, in the same order of sums. The gathered form keeps a row (58 doubles) and its unknowns in
+// registers, 184 to 210 a thread, one CTA of 256 an SM: while one such wave covers the lattice (WAVE, up to
+// ROW_WAVE nodes) the round trip is all that counts, past it the CTAs in flight do. A launch of k_pcg_matvec
+// with a cold L2, gathered and not, us: 128 x 128 14.3 and 18.4, 192 x 192 16.3 and 18.7, 224 x 224 22.0 and
+// 20.5, 256 x 256 23.1 and 20.8, 384 x 384 39.7 and 29.2, 500 x 500 55.6 and 44.3.
+constexpr int ROW_WAVE = 148 * 256;
+template <bool WAVE, class X, class XAt>
+__device__ __forceinline__ void pcgRow(const DLevel& F, const double2* __restrict__ op64, int n, XAt xAt, double& y0, double& y1, double& y2) {
+  if constexpr (WAVE)
+    pcgRowGather<X>(F, op64, n, xAt, y0, y1, y2);
+  else
+    pcgRowApply<X>(F, op64, n, xAt, y0, y1, y2);
+}
+
 // The same residual from the FP64 fine rows (the operator PCG solves with), every product and sum in
 // FP64: on torn cloth the FP32 row's stiff terms cancel on a loose strand's rigid motion only to ~6e-8
 // of their size, which is larger than the strand's inertia, so the V-cycle would restrict noise there.
-__global__ void k_residual_fine64(DLevel F, const double2* __restrict__ op64) {
+template <bool WAVE>
+__global__ void __launch_bounds__(128, WAVE ? 1 : 8) k_residual_fine64(DLevel F, const double2* __restrict__ op64) {
   pdlWait();
   pdlLaunchNext();
   int n = blockIdx.x * blockDim.x + threadIdx.x;
@@ -317,11 +360,12 @@ __global__ void k_residual_fine64(DLevel F, const double2* __restrict__ op64) {
   const uint32_t fixedRow = F.fixed[n];
   const float4 b = F.B[n];
   double y0 = 0.0, y1 = 0.0, y2 = 0.0;
-  pcgRowGather<float>(
+  pcgRow<WAVE, float>(
       F, op64, n,
       [&](int q, float* x) {
         const float4 v = F.X[q];
         x[0] = v.x, x[1] = v.y, x[2] = v.z;
+        return true;
       },
       y0, y1, y2);
   F.R[n] = fixedRow ? make_float4(0, 0, 0, 0) : make_float4((float)(b.x - y0), (float)(b.y - y1), (float)(b.z - y2), 0.f);

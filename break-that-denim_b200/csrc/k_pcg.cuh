@@ -136,34 +136,6 @@ __global__ void __launch_bounds__(RED_THREADS) k_pcg_init(PcgArgs a) {
   }
 }
 
-// y += (row n of the operator PCG solves with) x, in FP64: the FP64 row when there is one, else the fp32
-// row's products summed in FP64. xAt(m, q) puts node m's x in q and returns false for a node whose x is
-// zero (skipped).
-template <class XAt>
-__device__ __forceinline__ void pcgRowApply(const PcgArgs& a, int n, XAt xAt, double& y0, double& y1, double& y2) {
-  const DLevel& F = a.F;
-  int i, j, l;
-  nodeAt(F, n, &i, &j, &l);
-  const DLevelLayer L = layerOf(F, l);
-  double q[3];
-  if (xAt(n, q)) {
-    if (a.op64)
-      symDVecAdd(loadSymD(a.op64, F.N, n, 0), q, y0, y1, y2);
-    else
-      symVecAddD(FineRows::diag(F.op, F.N, n), q, y0, y1, y2);
-  }
-#pragma unroll
-  for (int k = 0; k < FineRows::NC; ++k) {
-    const int2 off = FineRows::offset(k);
-    const int m = levelNode(L, i + off.x, j + off.y);
-    if (m < 0 || !xAt(m, q)) continue;
-    if (a.op64)
-      symDVecAdd(fine64Block(a.op64, F.N, n, k), q, y0, y1, y2);
-    else
-      symVecAddD(FineRows::coupling(F.op, F.N, n, k), q, y0, y1, y2);
-  }
-}
-
 // The PCG start from the detached pieces' rigid modes (encodeRigidStart, solver.ts:651-657): delta = x0
 // (t + w x r on each piece's nodes, zero elsewhere), r = b - A x0 in FP64 (fixed rows 0), z = 0.
 __global__ void __launch_bounds__(RED_THREADS) k_pcg_init_rigid(PcgArgs a, StepArgs S, RigidArgs R) {
@@ -181,8 +153,8 @@ __global__ void __launch_bounds__(RED_THREADS) k_pcg_init_rigid(PcgArgs a, StepA
     float3 r = make_float3(0, 0, 0);
     if (!F.fixed[n]) {
       double y0 = 0.0, y1 = 0.0, y2 = 0.0;
-      pcgRowApply(
-          a, n,
+      pcgRowApply<double>(
+          F, a.op64, n,
           [&](int m, double* q) {
             if (!inPiece(R, m)) return false;
             const Dv xm = rigidStartAt(S, R, m);
@@ -243,8 +215,9 @@ __global__ void __launch_bounds__(RED_THREADS) k_pcg_dot_rz(PcgArgs a, int first
 
 // p = z + beta p (first: p = z); Ap = A p (fixed rows 0), p . Ap; alpha = rz / pAp (0 and stop when
 // pAp <= 0, as pcg() breaks). Each node forms its neighbours' p as they do (one launch and one pass over p
-// less than an update of its own), so the new p goes to the other of two buffers.
-__global__ void __launch_bounds__(RED_THREADS) k_pcg_matvec(PcgArgs a, int first) {
+// less than an update of its own), so the new p goes to the other of two buffers. WAVE: see pcgRow.
+template <bool WAVE>
+__global__ void __launch_bounds__(RED_THREADS, WAVE ? 1 : 4) k_pcg_matvec(PcgArgs a, int first) {
   pdlWait();
   pdlLaunchNext();
   double v[1] = {0.0};
@@ -265,12 +238,13 @@ __global__ void __launch_bounds__(RED_THREADS) k_pcg_matvec(PcgArgs a, int first
     // stored Ap only
     double y0 = 0.0, y1 = 0.0, y2 = 0.0;
     float3 p;
-    pcgRowGather<float>(
+    pcgRow<WAVE, float>(
         F, a.op64, n,
         [&](int m, float* q) {
           const float3 pm = direction(m);
           if (m == n) p = pm;
           q[0] = pm.x, q[1] = pm.y, q[2] = pm.z;
+          return true;
         },
         y0, y1, y2);
     if (!fixedRow) y = make_float3((float)y0, (float)y1, (float)y2);
@@ -354,7 +328,8 @@ __global__ void __launch_bounds__(RED_THREADS) k_pcg_update_xr(PcgArgs a) {
 // recurrence drifted): r replaces the recurrence residual (stored fp32) and the next direction starts
 // afresh (keeping the old one stalls: measured ~10x more iterations), so the fp32 iterations solve
 // for a correction that accumulates into the FP64 iterate - iterative refinement.
-__global__ void __launch_bounds__(RED_THREADS) k_pcg_true_residual(PcgArgs a) {
+template <bool WAVE>
+__global__ void __launch_bounds__(RED_THREADS, WAVE ? 1 : 4) k_pcg_true_residual(PcgArgs a) {
   pdlWait();
   pdlLaunchNext();
   if (!a.scal->check) return;
@@ -364,8 +339,13 @@ __global__ void __launch_bounds__(RED_THREADS) k_pcg_true_residual(PcgArgs a) {
     const float3 b = f3(a.b0[n]);
     double y0 = 0.0, y1 = 0.0, y2 = 0.0;
     const uint32_t fixedRow = F.fixed[n];
-    pcgRowGather<double>(
-        F, a.op64, n, [&](int m, double* q) { q[0] = a.dd[3 * m], q[1] = a.dd[3 * m + 1], q[2] = a.dd[3 * m + 2]; }, y0, y1, y2);
+    pcgRow<WAVE, double>(
+        F, a.op64, n,
+        [&](int m, double* q) {
+          q[0] = a.dd[3 * m], q[1] = a.dd[3 * m + 1], q[2] = a.dd[3 * m + 2];
+          return true;
+        },
+        y0, y1, y2);
     if (fixedRow) y0 = y1 = y2 = 0.0;
     const double r0 = (double)b.x - y0, r1 = (double)b.y - y1, r2 = (double)b.z - y2;
     a.F.B[n] = make_float4((float)r0, (float)r1, (float)r2, 0.f);

@@ -690,6 +690,9 @@ struct btd_solver {
     tailFrom = from;
   }
 
+  // the fine rows' kernels in their gathered form (pcgRow)
+  bool rowWave() const { return N <= ROW_WAVE; }
+
   // encodeVCycle (solver.ts:584-598): X of level k = V(B) with X zero on entry.
   void encVCycle(cudaStream_t s, int k) {
     int last = (int)levels.size() - 1;
@@ -719,7 +722,7 @@ struct btd_solver {
     Level& Cl = levels[k + 1];
     encSmooth(s, k, false);
     if (F.fine && opFp64)
-      launch(k_residual_fine64, blocksFor(F.N, 128), 128, 0, s, F.dev(), (const double2*)op64);
+      launch(rowWave() ? k_residual_fine64<true> : k_residual_fine64<false>, blocksFor(F.N, 128), 128, 0, s, F.dev(), (const double2*)op64);
     else if (F.fine)
       launch(k_residual_fine, blocksFor(F.N, 128), 128, 0, s, F.dev());
     else
@@ -733,9 +736,9 @@ struct btd_solver {
   void encPcgBody(cudaStream_t s, const PcgArgs& a) {
     encVCycle(s, 0);
     launch(k_pcg_dot_rz, redBlocks, RED_THREADS, 0, s, a, 0);
-    launch(k_pcg_matvec, redBlocks, RED_THREADS, 0, s, a, 0);
+    launch(rowWave() ? k_pcg_matvec<true> : k_pcg_matvec<false>, redBlocks, RED_THREADS, 0, s, a, 0);
     launch(k_pcg_update_xr, redBlocks, RED_THREADS, 0, s, a);
-    launch(k_pcg_true_residual, redBlocks, RED_THREADS, 0, s, a);
+    launch(rowWave() ? k_pcg_true_residual<true> : k_pcg_true_residual<false>, redBlocks, RED_THREADS, 0, s, a);
   }
 
   // encodePCG (solver.ts:625-644) with the device-side stop: prologue, then a while-node whose
@@ -756,9 +759,9 @@ struct btd_solver {
     encPcgInit(s, a);
     encVCycle(s, 0);
     launch(k_pcg_dot_rz, redBlocks, RED_THREADS, 0, s, a, 1);
-    launch(k_pcg_matvec, redBlocks, RED_THREADS, 0, s, a, 1);
+    launch(rowWave() ? k_pcg_matvec<true> : k_pcg_matvec<false>, redBlocks, RED_THREADS, 0, s, a, 1);
     launch(k_pcg_update_xr, redBlocks, RED_THREADS, 0, s, a);
-    launch(k_pcg_true_residual, redBlocks, RED_THREADS, 0, s, a);
+    launch(rowWave() ? k_pcg_true_residual<true> : k_pcg_true_residual<false>, redBlocks, RED_THREADS, 0, s, a);
     CK(cudaStreamGetCaptureInfo(s, &st, nullptr, &g, &deps, &nDeps));
     cudaGraphNodeParams cp = {cudaGraphNodeTypeConditional};
     cp.conditional.handle = h;
@@ -781,9 +784,9 @@ struct btd_solver {
     encPcgInit(s, a);
     encVCycle(s, 0);
     launch(k_pcg_dot_rz, redBlocks, RED_THREADS, 0, s, a, 1);
-    launch(k_pcg_matvec, redBlocks, RED_THREADS, 0, s, a, 1);
+    launch(rowWave() ? k_pcg_matvec<true> : k_pcg_matvec<false>, redBlocks, RED_THREADS, 0, s, a, 1);
     launch(k_pcg_update_xr, redBlocks, RED_THREADS, 0, s, a);
-    launch(k_pcg_true_residual, redBlocks, RED_THREADS, 0, s, a);
+    launch(rowWave() ? k_pcg_true_residual<true> : k_pcg_true_residual<false>, redBlocks, RED_THREADS, 0, s, a);
     for (;;) {
       int conv = 0;
       CK(cudaMemcpyAsync(&conv, &dScal->converged, sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -2048,7 +2051,10 @@ int btd_profile_stage(btd_solver* s, int32_t which, int32_t reps, int32_t flush,
       CK(cudaEventRecord(e0, s->stream));
       switch (which) {
         case BTD_STAGE_MATVEC:
-          k_pcg_matvec<<<s->redBlocks, RED_THREADS, 0, s->stream>>>(pa, 0);
+          if (s->rowWave())
+            k_pcg_matvec<true><<<s->redBlocks, RED_THREADS, 0, s->stream>>>(pa, 0);
+          else
+            k_pcg_matvec<false><<<s->redBlocks, RED_THREADS, 0, s->stream>>>(pa, 0);
           break;
         case BTD_STAGE_SMOOTH:
           s->encSmooth(s->stream, 0, false);
