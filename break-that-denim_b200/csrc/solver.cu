@@ -495,12 +495,13 @@ struct btd_solver {
     }
   }
 
-  // Line factors of level k, every line of a family in one launch (after its operator changed).
+  // Line factors of level k (after its operator changed): every line in one launch, or a launch a family when
+  // one family is short enough for the compact sweep and the other is not.
   void encFactor(cudaStream_t s, int k) {
     Level& L = levels[k];
     const int split = L.colourStart[3], all = (int)L.lines.size();  // v-lines, then u-lines
-    if (L.compact(0) && L.compact(1)) {
-      encFactorLines(s, L, 0, all, L.maxLine, true);
+    if (L.compact(0) == L.compact(1)) {
+      encFactorLines(s, L, 0, all, L.maxLine, L.compact(0));
     } else {
       encFactorLines(s, L, 0, split, L.famLine[1], L.compact(1));
       encFactorLines(s, L, split, all - split, L.famLine[0], L.compact(0));
