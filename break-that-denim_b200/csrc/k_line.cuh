@@ -357,8 +357,15 @@ __global__ void __launch_bounds__(CUT_FACTOR_THREADS, 3) k_line_compact(DLevel L
   __syncthreads();
 
   // ---- the cut
-  for (int k = tid; k < len; k += nt) sE[k] = lineShift([&](int q, int d) { return sB[6 * q + (d == 0 ? 0 : d == 1 ? 3 : 5)]; },
-                                                             [&](int q, int d) { return sC[6 * q + (d == 0 ? 0 : d == 1 ? 3 : 5)]; }, k);
+  float* piv = reinterpret_cast<float*>(sF);  // not in use yet
+  for (int k = tid; k < len; k += nt) {
+    const float *B = sB + 6 * k, *C = sC + 6 * k;
+    piv[k] = B[0], piv[len + k] = B[3], piv[2 * len + k] = B[5];
+    piv[3 * len + k] = C[0] * C[0], piv[4 * len + k] = C[3] * C[3], piv[5 * len + k] = C[5] * C[5];
+  }
+  __syncthreads();
+  linePivots(piv, len);
+  for (int k = tid; k < len; k += nt) sE[k] = lineShift(piv, len, k);
   __syncthreads();
   auto row = [&](int k) {
     M3d B = m3dSym(sB + 6 * k);

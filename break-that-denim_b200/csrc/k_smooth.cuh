@@ -270,22 +270,34 @@ struct Chunks {
 // (PIVOT_SHIFT). On a line's softest modes (inertia against spans 1e5 times stiffer) the shifts are of the
 // size of the matrix itself, so they have to be those of the reference's elimination along the line and not of
 // the partition's own pivots, which start every chunk anew: with those a sweep was 5e-4 from the FP64 oracle's,
-// with these it is 2e-5. The pivot's diagonal is followed entry by entry, s_k = B_k - A_k^2 / s_{k-1}, over the
-// LINE_BACK nodes before k; B(q, d) and A(q, d) are diagonal entry d of row q and of the block between q and q + 1.
-constexpr int LINE_BACK = 64;
-template <class GetB, class GetA>
-__device__ __forceinline__ float lineShift(GetB B, GetA A, int k) {
-  const int q0 = max(0, k - LINE_BACK);
-  float s[3] = {B(q0, 0), B(q0, 1), B(q0, 2)};
+// with these it is 2e-5. The pivot's diagonal is followed entry by entry, s_k = B_k - A_k^2 / s_{k-1}, over at
+// least the LINE_BACK nodes before k. A thread follows one entry over those nodes and then over a run of
+// LINE_RUN nodes or more (an odd number, so that the threads' reads fall in distinct banks). It is bound by the
+// chain of divisions, about 70 of them; a thread a node, with LINE_BACK steps of its own, did 14 times as many
+// and was bound by their number: assembly and fine factors of 150 x 150 nodes 124 us and now 116, 256 x 256 257
+// and 232, 384 x 384 515 and 435, 500 x 500 814 and 690.
+constexpr int LINE_BACK = 64, LINE_RUN = 5;
+// d: nine planes of len floats in shared memory - the diagonal entries of rows k (0 to 2) and the squares of
+// those of the block between k and k + 1 (3 to 5), and the pivots' entries, written here (6 to 8). The whole
+// CTA calls it; it ends with a barrier.
+__device__ __forceinline__ void linePivots(float* d, int len) {
+  const int perEntry = (int)blockDim.x / 3, run = max(LINE_RUN, (len + perEntry - 1) / perEntry) | 1, runs = (len + run - 1) / run;
+  for (int w = threadIdx.x; w < 3 * runs; w += blockDim.x) {
+    const int c = w / runs, k0 = (w - c * runs) * run, end = min(k0 + run, len);
+    const float *B = d + c * len, *A2 = d + (3 + c) * len;
+    float* out = d + (6 + c) * len;
+    int q = max(0, k0 - LINE_BACK);
+    float s = B[q];
+    auto step = [&](int k) { s = fmaxf(B[k] - __fdividef(A2[k - 1], s), 1e-3f * B[k]); };
 #pragma unroll 8
-  for (int q = q0 + 1; q <= k; ++q) {
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      const float b = B(q, d), a = A(q - 1, d);
-      s[d] = fmaxf(b - __fdividef(a * a, s[d]), 1e-3f * b);
-    }
+    for (++q; q <= k0; ++q) step(q);
+    out[k0] = s;
+    for (q = k0 + 1; q < end; ++q) step(q), out[q] = s;
   }
-  return 2e-6f * fmaxf(fmaxf(s[0], s[1]), s[2]);
+  __syncthreads();
+}
+__device__ __forceinline__ float lineShift(const float* d, int len, int k) {
+  return 2e-6f * fmaxf(fmaxf(d[6 * len + k], d[7 * len + k]), d[8 * len + k]);
 }
 
 // ------------------------------------------------------------------------------------------ factor
@@ -369,20 +381,17 @@ __global__ void __launch_bounds__(SM_THREADS) k_line_factor(DLevel L, const int4
     sF[2 * NP + ch.idx(k)] = make_float4(0.f, maj, L.fixed[n] != 0u ? 1.f : 0.f, 0.f);
   }
   __syncthreads();
-  // ---- the rows' shifts, found before any is added
-  auto diagonal = [](const float4* p, int d) { return d == 0 ? p[0].x : d == 1 ? p[0].w : p[1].y; };
-  float shift[(SM_MAX_LINE + SM_THREADS - 1) / SM_THREADS];
-#pragma unroll
-  for (int q = 0; q < (SM_MAX_LINE + SM_THREADS - 1) / SM_THREADS; ++q) {
-    const int k = tid + q * SM_THREADS;
-    shift[q] = k < len ? lineShift([&](int r, int d) { return diagonal(sB + 2 * r, d); }, [&](int r, int d) { return diagonal(sC + 2 * r, d); }, k) : 0.f;
+  // ---- the rows' shifts (the staging columns' space is free)
+  static_assert(4 * PL * SM_THREADS >= 9 * SM_MAX_LINE, "the pivots' planes");
+  float* piv = reinterpret_cast<float*>(cols);
+  for (int k = tid; k < len; k += SM_THREADS) {
+    const Sym Bk = ldS(sB + 2 * k), Ck = ldS(sC + 2 * k);
+    piv[k] = Bk.xx, piv[len + k] = Bk.yy, piv[2 * len + k] = Bk.zz;
+    piv[3 * len + k] = Ck.xx * Ck.xx, piv[4 * len + k] = Ck.yy * Ck.yy, piv[5 * len + k] = Ck.zz * Ck.zz;
   }
   __syncthreads();
-#pragma unroll
-  for (int q = 0; q < (SM_MAX_LINE + SM_THREADS - 1) / SM_THREADS; ++q) {
-    const int k = tid + q * SM_THREADS;
-    if (k < len) stS(sB + 2 * k, ldS(sB + 2 * k) + symId(shift[q]));
-  }
+  linePivots(piv, len);
+  for (int k = tid; k < len; k += SM_THREADS) stS(sB + 2 * k, ldS(sB + 2 * k) + symId(lineShift(piv, len, k)));
   __syncthreads();
 
   // ---- chunk interiors: Minv, Minv A, G; then V, W by the backward pass; reduced rows. Node k of
