@@ -280,6 +280,7 @@ struct btd_solver {
   // While a substep of a batch is captured: its coarse levels keep their launches, as a cluster needs sixteen
   // SMs of one GPC at once that the other patches' lines are on. The arithmetic is the same bit for bit.
   bool batched = false;
+  bool ranBatched = false;  // the last substeps ran so (btd_launch_count)
   // the levels from here down run as one cluster launch (k_tail; -1: none)
   int tailFrom = -1;
   TailVisit* dTailVisits = nullptr;
@@ -959,6 +960,7 @@ struct btd_solver {
   }
   void runSubstep(int minIterations, int maxIterations) {
     const int iters = unconditional(minIterations), itersMax = gatedBound(minIterations, maxIterations);
+    ranBatched = false;
     if (useGraphs)
       CK(cudaGraphLaunch(substepGraph(iters, itersMax), stream));
     else
@@ -1355,6 +1357,7 @@ int btd_substeps(btd_solver* s, int32_t count) {
       for (int k = 0; k < count; ++k) s->runSubstepEager(s->unconditional(0), s->gatedBound(0, 0));
     } else {
       cudaGraphExec_t ex = s->substepGraph(s->unconditional(0), s->gatedBound(0, 0));
+      s->ranBatched = false;
       for (int k = 0; k < count; ++k) CK(cudaGraphLaunch(ex, s->stream));
     }
   });
@@ -1368,6 +1371,7 @@ int btd_batch_substeps(btd_solver* const* solvers, int32_t count, int32_t subste
       btd_solver* s = solvers[b];
       checkSolver(s);
       if (s->useGraphs) graphs[b] = s->substepGraph(s->unconditional(0), s->gatedBound(0, 0), count > 1);
+      s->ranBatched = s->useGraphs && count > 1;
     }
     // round robin: every patch's next substep is queued before any patch's one after, so all
     // streams have work from the start
@@ -1497,7 +1501,10 @@ int btd_batch_run(btd_batch* b, int32_t substeps) {
       }
       CK(cudaGraphLaunch(b->exec, b->stream));
       CK(cudaEventRecord(b->join, b->stream));
-      for (btd_solver* s : b->solvers) CK(cudaStreamWaitEvent(s->stream, b->join, 0));
+      for (btd_solver* s : b->solvers) {
+        CK(cudaStreamWaitEvent(s->stream, b->join, 0));
+        s->ranBatched = true;
+      }
     }
   });
 }
@@ -2097,9 +2104,12 @@ int btd_launch_count(btd_solver* s, int32_t substeps, int32_t newton, int32_t pc
     };
     const int L = (int)s->levels.size();
     const int64_t lc = s->lcOn() ? 1 : 0;
-    const int tail = s->tailFrom >= 0 ? s->tailFrom : L - 1;  // from here down one launch, two around the learned correction
-    int64_t V = (s->tailFrom >= 0 ? 1 + lc : s->params.coarse_sweeps * colours(L - 1)) + lc;
+    // from the cluster launch's first level down one launch, two around the learned correction; not in a batch
+    const bool clustered = s->tailFrom >= 0 && !s->ranBatched;
+    const int tail = clustered ? s->tailFrom : L - 1;
+    int64_t V = (clustered ? 1 + lc : s->params.coarse_sweeps * colours(L - 1)) + lc;
     for (int k = 0; k < tail; ++k) V += 2 * colours(k) + 3;
+    auto factors = [&](int k) -> int64_t { return s->levels[k].compact(0) == s->levels[k].compact(1) ? 1 : 2; };
     // per Newton iteration: assembly, PCG prologue (init + V-cycle + 4), line search, apply; the
     // hierarchy (weights + RAP per coarse level) on the first iteration; V-cycle + 4 per extra PCG pass
     // held grips add their lead once per substep and their terms once per Newton iteration; the
@@ -2112,13 +2122,14 @@ int btd_launch_count(btd_solver* s, int32_t substeps, int32_t newton, int32_t pc
     const int64_t rigid = s->pieceCount > 0 ? 1 : 0;
     const int64_t xc = s->xcOn() ? 1 : 0;  // cross-layer contact: terms in one kernel, detection in five
     // the learned correction adds its flags (fine, then one a coarse level) and basis to every solve
-    const int64_t perNewton = 2 + (1 + V + 4) + 1 + 1 + grips + (2 - xc) * contact + 4 * rigid + lc * (L + 1);
-    const int64_t hierarchy = 3 * (L - 1);
-    const int64_t hierPerSubstep = s->params.lag_coarse ? hierarchy : hierarchy * (newton / std::max(1, substeps));
+    const int64_t perNewton = 1 + factors(0) + (1 + V + 4) + 1 + 1 + grips + (2 - xc) * contact + 4 * rigid + lc * (L + 1);
+    int64_t hierarchy = lc;  // it marks the coarsest operator as new
+    for (int k = 1; k < L; ++k) hierarchy += 2 + factors(k);
+    const int64_t hierarchies = s->params.lag_coarse ? substeps : newton;
     const int64_t perSubstep = 2 + 1 + 5 + s->nLayers + 4 + grips + (7 - 2 * xc) * contact + 2 * rigid;
     // each optional (gated) Newton iteration slot adds its gate kernel, run or not
     const int64_t gates = s->gatedBound(0, 0) - s->unconditional(0);
-    *out = (int64_t)substeps * (perSubstep + hierPerSubstep + gates) + (int64_t)newton * perNewton + (int64_t)(pcg - newton) * (V + 4);
+    *out = (int64_t)substeps * (perSubstep + gates) + hierarchies * hierarchy + (int64_t)newton * perNewton + (int64_t)(pcg - newton) * (V + 4);
   });
 }
 

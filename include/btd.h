@@ -363,7 +363,8 @@ int btd_read_grip(btd_solver* s, int32_t slot, int32_t* nodes, float* weights, i
 #define BTD_STAGE_SUBSTEP 5 /* a whole substep: one launch of the captured substep graph */
 int btd_profile_stage(btd_solver* s, int32_t which, int32_t reps, int32_t flush, float* ms_per_launch);
 /* Kernel launches of substeps that ran `newton_iterations` Newton iterations and `pcg_iterations`
- * PCG iterations in total (the graph's nodes that are kernels, loop bodies counted per pass). */
+ * PCG iterations in total (the graph's nodes that are kernels, loop bodies counted per pass), as the solver's
+ * last substeps ran: alone, or in a batch, where the coarse levels take a launch a colour. */
 int btd_launch_count(btd_solver* s, int32_t substeps, int32_t newton_iterations, int32_t pcg_iterations, int64_t* out);
 /* Autotuner of the yarn-line sweeps' launch shapes (no counterpart in the reference, whose workgroup
  * size is fixed at 128, smooth.wgsl:86): for every multigrid level the CTA size (multiples of 32 from 64

@@ -33,3 +33,48 @@ def test_a_level_is_factored_in_one_launch_unless_its_families_take_different_ke
     assert sum("k_assemble" in n for n in names) == 1  # the trace sees the library
     assert sum("k_line_" in n for n in names) == launches, names
     g.close()
+
+
+def counted(g):
+    c = g.counter_dict()
+    return g.launch_count(1, c["newton"], c["pcg_total"])
+
+
+@pytest.mark.parametrize("kind", ["plain", "mixed", "rebuilt", "learned"])
+def test_launch_count_is_the_kernels_of_a_substep(kind):
+    if kind == "learned":  # grips, self-contact and the learned correction
+        sc, left, _ = btd.configs.config4(n=64, region=16)
+        g = btd.GpuSolver(sc, btd.configs.solver_params(1 / 120, 2, 1e-6, self_contact=1))
+        g.set_learned(btd.learned.load(), on=True, guard=0.9)
+        g.attach_patch(0, int(left[0]), left, np.ones(len(left)), g.x[left[0]], 500.0, max_lead=1.0)
+    else:
+        g = solver((160, 48) if kind == "mixed" else (64, 64), lag_coarse=0 if kind == "rebuilt" else 1)
+    g.set_graph_mode(False)
+    g.substep()
+    g.clear_counters()
+    names = kernels(g.substep, g.synchronize)
+    assert len(names) == counted(g)
+    g.close()
+
+
+def test_launch_count_of_a_batch():
+    """In a batch the V-cycle's coarse levels take a launch a colour (six) in place of the one cluster launch: two
+    sweeps of each, the coarsest included, and a residual, a restriction and a prolongation between two of them."""
+    solvers = [solver((64, 64)), solver((36, 20))]
+    assert [g.level_count() for g in solvers] == [3, 2]
+    for g in solvers:
+        g.substep()
+    alone = [g.launch_count(1, 2, 20) for g in solvers]
+    batch = btd.Batch(solvers)
+    batch.run(1)
+    for g in solvers:
+        g.synchronize()
+    # levels in the cluster launch: 33 x 33 and 17 x 17 nodes; 18 x 10 nodes
+    for g, before, own in zip(solvers, alone, (12 + 3 + 12, 12)):
+        assert g.launch_count(1, 2, 20) - before == 20 * (own - 1)
+    for g in solvers:
+        g.substep()
+    assert [g.launch_count(1, 2, 20) for g in solvers] == alone
+    batch.close()
+    for g in solvers:
+        g.close()
