@@ -147,9 +147,10 @@ __device__ __forceinline__ bool mbarTryWait(uint64_t* bar, unsigned parity) {
 // Bounded wait for phase `parity` of an mbarrier (each try suspends the thread for a while). If the
 // first bound runs out, the error flag is raised and the wait gets a second bound of its own, so that
 // copies still in flight land before the CTA goes on and exits; either way the kernel goes on (with
-// garbage, flagged) instead of hanging. The copies waited on are this CTA's own bulk copies from
-// global memory (tens of KB, microseconds), so the second bound (2^20 tries, seconds) runs out only
-// when the expected transaction bytes exceed the bytes issued - a bug, with no copy left in flight.
+// garbage, flagged) instead of hanging. The second bound (2^20 tries, seconds) runs out only for a bug.
+// k_smooth waits on its CTA's own bulk copies from global memory (tens of KB, microseconds): then the
+// expected bytes exceed the bytes issued and no copy is left in flight. k_tail waits on what other CTAs
+// send, and sees to it that none leaves before the others (see there).
 // The first bound is a device variable so that a test can make it run out (btd_set_wait_bound): with
 // zero tries the flag is raised at once and the copies land under the second bound.
 constexpr int MBAR_TRIES = 1 << 20;

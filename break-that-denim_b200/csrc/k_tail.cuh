@@ -11,7 +11,10 @@
 //
 // Every CTA sends in every exchange (one without a line sends a 16-byte token), so no CTA can be more than
 // one exchange ahead of another: two mbarriers in turn suffice, and what a CTA reads of its copy before it
-// sends is not overwritten under it. The waits are bounded (mbarWaitBounded).
+// sends is not overwritten under it. The waits are bounded (mbarWaitBounded). A CTA whose wait runs out in both
+// bounds (a bug; its error flag is up) goes on without the turn that the others are at. So that nothing is then
+// sent to a CTA that has left, all leave together, after a barrier of the cluster (every CTA's way to it is
+// bounded; it costs nothing that can be measured, 101.8 us a V-cycle of 64 x 64 nodes with it and without).
 #pragma once
 
 #include "k_line.cuh"
@@ -56,6 +59,7 @@ __device__ __forceinline__ unsigned clusterRank() {
   return r;
 }
 __device__ __forceinline__ void clusterArrive() { asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory"); }
+__device__ __forceinline__ void clusterArriveRelaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;\n" ::: "memory"); }
 __device__ __forceinline__ void clusterWait() { asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory"); }
 __device__ __forceinline__ unsigned mapaOf(unsigned addr, unsigned rank) {
   unsigned r;
@@ -302,6 +306,7 @@ __global__ void __launch_bounds__(TAIL_THREADS, 1) k_tail(TailArgs a) {
     }
   }
   __syncthreads();
+  clusterArriveRelaxed();
   // the levels' vectors, as the launches of every step would leave them: for the learned correction, the
   // resumed call and readers
   for (int l = 0; l < a.levels; ++l) {
@@ -312,6 +317,7 @@ __global__ void __launch_bounds__(TAIL_THREADS, 1) k_tail(TailArgs a) {
       if (L.b0 >= 0) L.d.B[n] = sm4[L.b0 + n];
     }
   }
+  clusterWait();
 }
 
 }  // namespace btd
