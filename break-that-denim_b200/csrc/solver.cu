@@ -11,6 +11,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstdlib>
 #include <cstring>
 #include <functional>
 #include <map>
@@ -280,6 +281,28 @@ struct btd_solver {
   // While a substep of a batch is captured: its coarse levels keep their launches, as a cluster needs sixteen
   // SMs of one GPC at once that the other patches' lines are on. The arithmetic is the same bit for bit.
   bool batched = false;
+  // Whether the patches of that batch that run side by side (the device's hardware queues hold as many branches) have
+  // more nodes than 2.5 waves of the row kernels: they then compete for the SMs, and the kernels that leave one CTA
+  // an SM to shorten a lone patch's chain (the gathered rows, the compact sweeps of fine lines over 72 nodes) give
+  // way to forms that leave more. A PCG iteration, us, with 32 queues: 32 patches of 128 x 128 36.1 -> 30.2, 24 of 96 x
+  // 96 22.2 -> 18.7, 12 of 182 x 182 68.7 -> 60.8, 24 of 64 x 64 11.9 -> 11.2; the line is where the two meet: 11 of
+  // 96 x 96 (101,376 nodes) 25.7 in both, 6 of 128 x 128 (98,304) 46.3 and 46.1, 5 of them (81,920) 51.2 and 52.9;
+  // with 8 queues 24 of 96 x 96 (73,728 at a time) 30.9 and 32.4, 24 of 16 to 128 a side (46,018) 49.8 and 52.5 ms.
+  static constexpr int64_t BATCH_CROWD = 5 * ROW_WAVE / 2;
+  bool crowded = false;
+  // A batch's nodes in flight.
+  static int64_t inFlight(btd_solver* const* solvers, size_t count) {
+    const char* q = std::getenv("CUDA_DEVICE_MAX_CONNECTIONS");  // 8 unless set
+    const int64_t queues = std::min(32, std::max(1, q ? std::atoi(q) : 8));
+    int64_t nodes = 0;
+    for (size_t b = 0; b < count; ++b) nodes += solvers[b]->N;
+    return (int64_t)count <= queues ? nodes : nodes * queues / (int64_t)count;
+  }
+  struct InBatch {
+    btd_solver& s;
+    InBatch(btd_solver& s_, int64_t nodes) : s(s_) { s.batched = nodes > 0, s.crowded = nodes > BATCH_CROWD; }
+    ~InBatch() { s.batched = s.crowded = false; }
+  };
   bool ranBatched = false;  // the last substeps ran so (btd_launch_count)
   // the levels from here down run as one cluster launch (k_tail; -1: none)
   int tailFrom = -1;
@@ -575,6 +598,8 @@ struct btd_solver {
       L.fine ? rows(k_sweep<FineRows, 1, 160, 3>, k_sweep<FineRows, 0, 160, 3>) : rows(k_sweep<CoarseRows, 1, 160, 3>, k_sweep<CoarseRows, 0, 160, 3>);
     else if (nt <= 288)
       L.fine ? rows(k_sweep<FineRows, 1, 288, 2>, k_sweep<FineRows, 0, 288, 2>) : rows(k_sweep<CoarseRows, 1, 288, 2>, k_sweep<CoarseRows, 0, 288, 2>);
+    else if (L.fine && crowded && nt <= 512)  // two CTAs an SM for a few spills (a lone sweep of 96 x 96 nodes: 24.3 us, 21.9 without)
+      rows(k_sweep<FineRows, 1, 512, 2>, k_sweep<FineRows, 0, 512, 2>);
     else
       L.fine ? rows(k_sweep<FineRows, 1, 544, 1>, k_sweep<FineRows, 0, 544, 1>) : rows(k_sweep<CoarseRows, 1, 544, 1>, k_sweep<CoarseRows, 0, 544, 1>);
   }
@@ -693,7 +718,7 @@ struct btd_solver {
   }
 
   // the fine rows' kernels in their gathered form (pcgRow)
-  bool rowWave() const { return N <= ROW_WAVE; }
+  bool rowWave() const { return N <= ROW_WAVE && !crowded; }
 
   // encodeVCycle (solver.ts:584-598): X of level k = V(B) with X zero on entry.
   void encVCycle(cudaStream_t s, int k) {
@@ -941,20 +966,14 @@ struct btd_solver {
     return std::min(MAX_NEWTON, std::max(std::max(params.newton_max, unconditional(minIterations)), maxIterations));
   }
 
-  cudaGraphExec_t substepGraph(int iters, int itersMax, bool inBatch = false) {
+  // `batchNodes`: in flight of the batch that the substep runs in (0: alone).
+  cudaGraphExec_t substepGraph(int iters, int itersMax, int64_t batchNodes = 0) {
     const bool grips = gripsOn();
-    const int key = ((iters * (MAX_NEWTON + 1) + itersMax) * 2 + (grips ? 1 : 0)) * 2 + (inBatch ? 1 : 0);
+    const int key = ((iters * (MAX_NEWTON + 1) + itersMax) * 2 + (grips ? 1 : 0)) * 3 + (batchNodes > BATCH_CROWD ? 2 : batchNodes > 0 ? 1 : 0);
     auto it = substepExec.find(key);
     if (it != substepExec.end()) return it->second;
-    batched = inBatch;
-    cudaGraphExec_t ex = nullptr;
-    try {
-      ex = capture([&](cudaStream_t s) { encSubstep(s, iters, itersMax, grips); });
-    } catch (...) {
-      batched = false;
-      throw;
-    }
-    batched = false;
+    const InBatch in(*this, batchNodes);
+    cudaGraphExec_t ex = capture([&](cudaStream_t s) { encSubstep(s, iters, itersMax, grips); });
     substepExec[key] = ex;
     return ex;
   }
@@ -1367,10 +1386,11 @@ int btd_batch_substeps(btd_solver* const* solvers, int32_t count, int32_t subste
   GUARD({
     if (!solvers || count < 0 || substeps < 0) throw std::invalid_argument("bad batch");
     std::vector<cudaGraphExec_t> graphs(count, nullptr);
+    for (int b = 0; b < count; ++b) checkSolver(solvers[b]);
+    const int64_t nodes = btd_solver::inFlight(solvers, count);
     for (int b = 0; b < count; ++b) {
       btd_solver* s = solvers[b];
-      checkSolver(s);
-      if (s->useGraphs) graphs[b] = s->substepGraph(s->unconditional(0), s->gatedBound(0, 0), count > 1);
+      if (s->useGraphs) graphs[b] = s->substepGraph(s->unconditional(0), s->gatedBound(0, 0), count > 1 ? nodes : 0);
       s->ranBatched = s->useGraphs && count > 1;
     }
     // round robin: every patch's next substep is queued before any patch's one after, so all
@@ -1415,17 +1435,12 @@ struct btd_batch {
     CK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeRelaxed));
     try {
       CK(cudaEventRecord(fork, stream));
+      const int64_t nodes = btd_solver::inFlight(solvers.data(), solvers.size());
       for (size_t b = 0; b < solvers.size(); ++b) {
         btd_solver* s = solvers[b];
         CK(cudaStreamWaitEvent(s->stream, fork, 0));
-        s->batched = true;
-        try {
-          s->encSubstep(s->stream, s->unconditional(0), s->gatedBound(0, 0), s->gripsOn());
-        } catch (...) {
-          s->batched = false;
-          throw;
-        }
-        s->batched = false;
+        const btd_solver::InBatch in(*s, nodes);
+        s->encSubstep(s->stream, s->unconditional(0), s->gatedBound(0, 0), s->gripsOn());
         CK(cudaEventRecord(done[b], s->stream));
         CK(cudaStreamWaitEvent(stream, done[b], 0));
       }

@@ -81,6 +81,52 @@ def test_batch_graph_equals_each_patch_alone():
         s.close()
 
 
+@pytest.mark.parametrize("shapes, crowded", [([(128, 128), (96, 131), (73, 112), (131, 97)] + 3 * [(128, 128)], True),
+                                             ([(128, 131), (73, 50)], False)])
+def test_large_batches_equal_their_patches_alone(shapes, crowded):
+    """Batches on both sides of 94,720 nodes side by side (at most eight patches: one a hardware queue), past which the
+    kernels that leave one CTA an SM give way to others: the long compact sweeps and the row kernels, the same
+    arithmetic bit for bit."""
+    assert (sum(a * b for a, b in shapes) > 94720) == crowded
+    scenes = [btd.configs.hanging_patch(s, 0.3 / 63 * (s[0] - 1), seed=k) for k, s in enumerate(shapes)]
+    batch, alone = ([btd.GpuSolver(sc, btd.configs.solver_params(1 / 60, 4, 1e-6)) for sc in scenes] for _ in range(2))
+    graph = btd.Batch(batch)
+    graph.run(2)
+    btd.batch_substeps(batch, 1)
+    for s, a in zip(batch, alone):
+        a.substeps(3)
+        assert np.array_equal(s.x, a.x)
+        assert s.counters()[17] == a.counters()[17]
+    graph.close()
+    for s in batch + alone:
+        s.close()
+
+
+@pytest.mark.parametrize("sweeps, coarsest", [(2, 400), (1, 400), (3, 30)])
+def test_the_learned_correction_between_clustered_levels_equals_the_launches(sweeps, coarsest):
+    """The cluster launch of the coarse levels is split around the learned correction, its vectors handed through
+    memory; in a batch the levels take a launch a colour: the same bit for bit."""
+    c = btd.configs.CONFIG4
+    solvers = []
+    for _ in range(2):
+        sc, left, _ = btd.configs.config4(n=64, region=16)
+        s = btd.GpuSolver(sc, btd.configs.solver_params(c["h"], 4, 1e-6, coarse_sweeps=sweeps, max_coarsest_nodes=coarsest))
+        s.set_learned(btd.learned.load(), on=True, guard=0.9)
+        picked = int(left[len(left) // 2])
+        s.attach_patch(0, picked, left, np.ones(len(left)), s.x[picked], c["grip_stiffness"], max_lead=1.0)
+        solvers.append(s)
+    small = btd.GpuSolver(btd.configs.hanging_patch(16, 0.07, seed=1), btd.configs.solver_params(1 / 60, 2, 1e-6))
+    graph = btd.Batch([solvers[0], small])
+    graph.run(3)
+    solvers[1].substeps(3)
+    assert np.array_equal(solvers[0].x, solvers[1].x)
+    assert solvers[0].counters()[17] == solvers[1].counters()[17]
+    assert solvers[1].learned_stats()["applied"] > 0
+    graph.close()
+    for s in solvers + [small]:
+        s.close()
+
+
 def test_batch_patches_match_the_oracle():
     """Three patches of the batch (their seeded sizes, stiffness factors, yarn regions and grips), run
     in the batch graph on the GPU and one by one in the oracle from the same float32 state: after 8
