@@ -759,9 +759,14 @@ def main():
     bytes_sweep = 2.0 * N * (R0 + 36.0)
     achieved = bytes_sweep / (ms_sweep / 1e3) / 1e9
     ms_mv = gpu.profile_stage("matvec", reps=10, flush=True)
-    # PCG's matvec reads the FP64 rows (58 doubles a node), p and the fixed flag, and writes Ap
+    # PCG's matvec reads the FP64 rows (58 doubles a node), z, the old direction and the fixed flag, and writes the new
+    # direction and Ap
     R64 = 464.0
-    mv_gbs = N * (R64 + 16.0 + 4.0 + 16.0) / (ms_mv / 1e3) / 1e9
+    mv_bytes = R64 + 16.0 + 16.0 + 4.0 + 16.0 + 16.0
+    mv_gbs = N * mv_bytes / (ms_mv / 1e3) / 1e9
+    # the fine sweep's kernels: families of lines up to 131 nodes take the compact one
+    kinds = {"k_sweep" if n <= 131 else "k_smooth" for n in (max(L.nx for L in sc.layers), max(L.ny for L in sc.layers))}
+    sweep_kernel = " and ".join(f"{k}<FineRows>" for k in sorted(kinds)) + " (fine yarn-line sweep, 6 colour launches)"
     traffic = None
     tpath = os.path.join(ROOT, "profiles", "traffic.json")
     if os.path.exists(tpath):
@@ -836,11 +841,11 @@ def main():
                 "loop": "each step: the state in from pinned host memory (the previous step's output), the grip targets, "
                         "one substep, the state out"},
         "gpu_launches": int(launches),
-        "roofline": {"kernel": "k_smooth<FineRows> (fine yarn-line sweep, 6 colour launches)", "bound": "hbm",
+        "roofline": {"kernel": sweep_kernel, "bound": "hbm",
                      "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak, "traffic": traffic,
                      "peak_kind": peak_kind, "algorithmic_bytes_per_sweep": bytes_sweep, "ms_per_sweep": ms_sweep,
                      "matvec_gbs": mv_gbs, "matvec_ms": ms_mv, "matvec_frac": mv_gbs / peak,
-                     "matvec_bytes_per_node": R64 + 36.0},
+                     "matvec_bytes_per_node": mv_bytes},
         "clocks": clocks.summary(),
     }
     line["config"]["levels"] = levels

@@ -7,9 +7,9 @@
 //                              those chunks' inverses, 3 rows of 2 Q floats)
 //   x_S = D rr                 D the inverse of the separators' Schur complement, dense
 //   x_I = C r_I + V x_l + W x_r  C the chunk's inverse, V and W its response to its two separators
-// three products with a barrier between them. k_line_compact forms E, D, C, V and W once per operator in
-// FP64 (pivots regularised as in k_line_factor) and stores them in FP32 in the order in which the sweep's
-// threads read them; k_sweep loads them - and its node's off-line couplings - into registers before the
+// three products with a barrier between them. k_line_compact forms D, C, V and W once per operator in
+// FP64 (rows regularised by lineShift, as in k_line_factor), and E from C as it is stored; it stores all in FP32
+// in the order in which the sweep's threads read them; k_sweep loads them - and its node's off-line couplings - into registers before the
 // grid-dependency wait, while the launch before it still runs.
 //
 // What bounds it: the dependent chain of one line and the boundary between two launches, not bytes (a coarse
@@ -18,8 +18,8 @@
 // 16 to 32 terms (0.45 us); the next launch's wait returns 1.1 us after the last store. A colour of a 64 x 64
 // lattice takes 2.6 us where k_smooth's took 3.3, and 2.9 where 3.5 at 128 x 128.
 //
-// The cut's line is the reference's to 2e-5 of a sweep's result (5e-4 for k_smooth's, whose pivots are shifted
-// chunk by chunk; see lineShift).
+// A sweep is 5e-7 to 1.3e-5 of its result from the FP64 oracle's on sheets at rest, as k_smooth's is, and 2e-5 to 6e-5
+// on a taut or torn patch (lineShift says what it is without the reference's shifts).
 #pragma once
 
 #include "k_smooth.cuh"
@@ -575,7 +575,8 @@ __device__ __forceinline__ float3 cutCouplings(const CutRegs<Rows>& R, const flo
 
 // The five columns of unknowns in shared memory: column a (0..4, the line's own 2) from a multiple of eight
 // float4 plus 2, 4, 6 for a = 1, 3, 4, so that the eight threads of a 128-bit access phase (two nodes, four
-// lanes, a column each) meet eight different bank groups.
+// lanes, a column each) meet eight different bank groups. Where len + 4 is a multiple of eight, the last two float4 of
+// column 1 are the first two of column 2: both are beyond the line's ends, zeros.
 __host__ __device__ constexpr int cutColumnStride(int len) { return (len + 4 + 7) / 8 * 8; }
 __host__ __device__ constexpr int cutColumn(int a, int len) {
   return a * cutColumnStride(len) + (a == 0 || a == 2 ? 0 : a == 1 ? 2 : a == 3 ? 4 : 6);

@@ -270,8 +270,9 @@ struct Chunks {
 // The shift that the reference's solve adds to row k of a line: 2e-6 of its pivot's largest diagonal entry
 // (PIVOT_SHIFT). On a line's softest modes (inertia against spans 1e5 times stiffer) the shifts are of the
 // size of the matrix itself, so they have to be those of the reference's elimination along the line and not of
-// the partition's own pivots, which start every chunk anew: with those a sweep was 5e-4 from the FP64 oracle's,
-// with these it is 2e-5. The pivot's diagonal is followed entry by entry, s_k = B_k - A_k^2 / s_{k-1}, over at
+// the partition's own pivots, which start every chunk anew: with those a sweep of a finest level was 8.5e-5 to 2e-4
+// from the FP64 oracle's on sheets at rest and 1.6e-4 to 8e-4 on a taut or torn patch, with these it is 9e-7 and 2e-5
+// to 6e-5. (PCG takes as many iterations with either: 190,783 and 186,688 over 256 substeps of a torn patch.) The pivot's diagonal is followed entry by entry, s_k = B_k - A_k^2 / s_{k-1}, over at
 // least the LINE_BACK nodes before k. A thread follows one entry over those nodes and then over a run of
 // LINE_RUN nodes or more (an odd number, so that the threads' reads fall in distinct banks). It is bound by the
 // chain of divisions, about 70 of them; a thread a node, with LINE_BACK steps of its own, did 14 times as many

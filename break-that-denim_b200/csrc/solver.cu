@@ -441,6 +441,7 @@ struct btd_solver {
       k_xc_count<<<blocksFor(N, 128), 128, 0, s>>>(a);
       encScan(s, xcCells, T);
       k_xc_fill<<<blocksFor(N, 128), 128, 0, s>>>(a);
+      k_xc_order<<<blocksFor(N, 128), 128, 0, s>>>(a);
       k_xc_detect<<<blocksFor(N, 128), 128, 0, s>>>(a, nLayers);
       return;
     }
@@ -2135,13 +2136,13 @@ int btd_launch_count(btd_solver* s, int32_t substeps, int32_t newton, int32_t pc
     const int64_t contact = s->contactOn() ? 1 : 0;
     // detached pieces add rotation + frame after the assembly, start (+ the init it replaces) and curves
     const int64_t rigid = s->pieceCount > 0 ? 1 : 0;
-    const int64_t xc = s->xcOn() ? 1 : 0;  // cross-layer contact: terms in one kernel, detection in five
+    const int64_t xc = s->xcOn() ? 1 : 0;  // cross-layer contact: terms in one kernel, detection in six
     // the learned correction adds its flags (fine, then one a coarse level) and basis to every solve
     const int64_t perNewton = 1 + factors(0) + (1 + V + 4) + 1 + 1 + grips + (2 - xc) * contact + 4 * rigid + lc * (L + 1);
     int64_t hierarchy = lc;  // it marks the coarsest operator as new
     for (int k = 1; k < L; ++k) hierarchy += 2 + factors(k);
     const int64_t hierarchies = s->params.lag_coarse ? substeps : newton;
-    const int64_t perSubstep = 2 + 1 + 5 + s->nLayers + 4 + grips + (7 - 2 * xc) * contact + 2 * rigid;
+    const int64_t perSubstep = 2 + 1 + 5 + s->nLayers + 4 + grips + (7 - xc) * contact + 2 * rigid;
     // each optional (gated) Newton iteration slot adds its gate kernel, run or not
     const int64_t gates = s->gatedBound(0, 0) - s->unconditional(0);
     *out = (int64_t)substeps * (perSubstep + gates) + hierarchies * hierarchy + (int64_t)newton * perNewton + (int64_t)(pcg - newton) * (V + 4);

@@ -371,8 +371,8 @@ int btd_launch_count(btd_solver* s, int32_t substeps, int32_t newton_iterations,
  * to 256) and, on lines longer than 128 nodes, the staging tile (whole line or 128 nodes) are timed on
  * the level's current operator (CUDA events, the mean of `reps` sweeps) and the fastest is kept for
  * every later sweep; results are unchanged bit for bit. A level whose lines are all short enough for the
- * compact sweep (131 nodes, 256 on the fine level) has a fixed shape, four threads a node: it is timed, and
- * its CTA size reported as 256 where it is more. Needs an assembled system (after a substep or
+ * compact sweep (131 nodes) has a fixed shape, four threads a node: it is timed, and its CTA size reported
+ * as 256 where it is more. Needs an assembled system (after a substep or
  * btd_stage_assemble). Per level (btd_level_count entries, any pointer may be NULL): the chosen CTA
  * size, tile, and the sweep's time in ms. */
 int btd_autotune(btd_solver* s, int32_t reps, int32_t* threads, int32_t* tile, float* ms);

@@ -130,3 +130,17 @@ def test_overlapping_mounted_plies_are_pushed_apart_like_the_oracle():
     free = sc.pinned == 0
     assert np.median(err[free]) < 0.01 * moved, (np.median(err[free]), moved)
     assert err.max() < 0.1 * moved, (err.max(), moved)
+
+
+def test_plies_that_touch_move_the_same_in_every_run():
+    """Two plies cut alike touch at many equal distances; which of them count must not depend on the order in which
+    threads reach a cell."""
+    m = btd.material_preset(0)
+    sc = btd.compile_scene([btd.layer_spec(m, 0.015, 0.015, bundle=(1, 1), z=z, seed=3) for z in (0.0, 0.5 * R)])
+    ends = []
+    for _ in range(6):
+        g = btd.GpuSolver(sc, btd.configs.solver_params(H, 4, 1e-6, pcg_cap=200, self_contact=1, cross_layer=1))
+        g.substeps(12)
+        ends.append(g.x.copy())
+        g.close()
+    assert all(np.array_equal(e, ends[0]) for e in ends)

@@ -40,13 +40,17 @@ def counted(g):
     return g.launch_count(1, c["newton"], c["pcg_total"])
 
 
-@pytest.mark.parametrize("kind", ["plain", "mixed", "rebuilt", "learned"])
+@pytest.mark.parametrize("kind", ["plain", "mixed", "rebuilt", "learned", "layers"])
 def test_launch_count_is_the_kernels_of_a_substep(kind):
     if kind == "learned":  # grips, self-contact and the learned correction
         sc, left, _ = btd.configs.config4(n=64, region=16)
         g = btd.GpuSolver(sc, btd.configs.solver_params(1 / 120, 2, 1e-6, self_contact=1))
         g.set_learned(btd.learned.load(), on=True, guard=0.9)
         g.attach_patch(0, int(left[0]), left, np.ones(len(left)), g.x[left[0]], 500.0, max_lead=1.0)
+    elif kind == "layers":  # contact between layers
+        m = btd.material_preset(0)
+        sc = btd.compile_scene([btd.layer_spec(m, 0.01, 0.01, bundle=(1, 1), z=z, seed=3) for z in (0.0, 3e-4)])
+        g = btd.GpuSolver(sc, btd.configs.solver_params(1 / 120, 2, 1e-6, pcg_cap=20, self_contact=1, cross_layer=1))
     else:
         g = solver((160, 48) if kind == "mixed" else (64, 64), lag_coarse=0 if kind == "rebuilt" else 1)
     g.set_graph_mode(False)
